@@ -17,6 +17,37 @@
 
 namespace bkg {
 
+// The even and the odd half of a line's contraction (EOMat, EORMat) run side
+// by side, one per lane: a coefficient pair C2 (even lane, odd lane), a value
+// pair V2 and an accumulator pair A2 per engine.  FP32-pipe engines hold them
+// packed (two lanes per instruction, bk_ff.cuh), the DFMA engine as two
+// doubles.
+template <class C>
+struct CoefPair;
+template <>
+struct CoefPair<double> {
+    double x, y;
+    void set(double a, double b)
+    {
+        x = a;
+        y = b;
+    }
+};
+template <>
+struct CoefPair<float> {
+    f2 v;
+    void set(float a, float b) { v = f2_make(a, b); }
+};
+template <>
+struct CoefPair<ff> : ffcp {
+    void set(ff a, ff b)
+    {
+        hi = f2_make(a.hi, b.hi);
+        nhi = f2_make(-a.hi, -b.hi);
+        lo = f2_make(a.lo, b.lo);
+    }
+};
+
 struct EngDfma {
     using S = double;
     using V = double;
@@ -38,14 +69,29 @@ struct EngDfma {
     __device__ static __forceinline__ V mul(V a, V b) { return a * b; }
     __device__ static __forceinline__ V vadd(V a, V b) { return a + b; }
     __device__ static __forceinline__ V vsub(V a, V b) { return a - b; }
-    __device__ static __forceinline__ V vadd_in(V a, V b) { return a + b; }
-    __device__ static __forceinline__ V vsub_in(V a, V b) { return a - b; }
-    __device__ static __forceinline__ void sum_diff(const A& a, const A& b, V& s, V& d)
+    struct V2 {
+        V x, y;
+    };
+    using A2 = V2;
+    // (a + b, a - b): the even and odd combinations of two line values
+    __device__ static __forceinline__ V2 even_odd(V a, V b) { return V2{a + b, a - b}; }
+    __device__ static __forceinline__ V even(const V2& v) { return v.x; }
+    __device__ static __forceinline__ V odd(const V2& v) { return v.y; }
+    __device__ static __forceinline__ A2 first2(const CoefPair<C>& c, const V2& v) { return A2{c.x * v.x, c.y * v.y}; }
+    __device__ static __forceinline__ void madd2(A2& acc, const CoefPair<C>& c, const V2& v)
     {
-        s = a + b;
-        d = b - a;
+        acc.x = fma(c.x, v.x, acc.x);
+        acc.y = fma(c.y, v.y, acc.y);
     }
-    __device__ static __forceinline__ void sum_diff_loose(const A& a, const A& b, V& s, V& d) { sum_diff(a, b, s, d); }
+    // the even lane alone
+    __device__ static __forceinline__ void madd_even(A2& acc, C c, V x) { acc.x = fma(c, x, acc.x); }
+    // s = even + odd; d = odd - even (SIGN < 0) or even - odd (SIGN > 0)
+    template <int SIGN, bool LOOSE>
+    __device__ static __forceinline__ void sum_diff(const A2& a, V& s, V& d)
+    {
+        s = a.x + a.y;
+        d = SIGN > 0 ? a.x - a.y : a.y - a.x;
+    }
     static C coef(double d) { return d; }
 };
 
@@ -73,15 +119,35 @@ struct EngFF {
     __device__ static __forceinline__ V mul(V a, V b) { return ff_mul(a, b); }
     __device__ static __forceinline__ V vadd(V a, V b) { return ff_add(a, b); }
     __device__ static __forceinline__ V vsub(V a, V b) { return ff_add(a, ff{-b.hi, -b.lo}); }
+    using V2 = ffp;
+    using A2 = ffaccp;
     // operands of multiply-adds only: not renormalised
-    __device__ static __forceinline__ V vadd_in(V a, V b) { return ff_add_loose(a, b); }
-    __device__ static __forceinline__ V vsub_in(V a, V b) { return ff_add_loose(a, ff{-b.hi, -b.lo}); }
-    // a + b and b - a of two accumulators
-    __device__ static __forceinline__ void sum_diff(const A& a, const A& b, V& s, V& d) { acc_sum_diff(a, b, s, d); }
-    // the same as unevaluated pairs, for outputs that are only summed next
-    __device__ static __forceinline__ void sum_diff_loose(const A& a, const A& b, V& s, V& d)
+    __device__ static __forceinline__ V2 even_odd(V a, V b)
     {
-        acc_sum_diff_loose(a, b, s, d);
+        return ffp_make(ff_add_loose(a, b), ff_add_loose(a, ff{-b.hi, -b.lo}));
+    }
+    __device__ static __forceinline__ V even(const V2& v) { return ffp_x(v); }
+    __device__ static __forceinline__ V odd(const V2& v) { return ffp_y(v); }
+    __device__ static __forceinline__ A2 first2(const CoefPair<C>& c, const V2& v) { return acc_first2(c, v); }
+    __device__ static __forceinline__ void madd2(A2& acc, const CoefPair<C>& c, const V2& v) { acc_madd2(acc, c, v); }
+    __device__ static __forceinline__ void madd_even(A2& acc, C c, V x)
+    {
+        ffacc a{f2_x(acc.s), f2_x(acc.c)};
+        acc_madd(a, c, x);
+        acc = A2{f2_make(a.s, f2_y(acc.s)), f2_make(a.c, f2_y(acc.c))};
+    }
+    // LOOSE: unevaluated pairs, for outputs that are only summed next
+    template <int SIGN, bool LOOSE>
+    __device__ static __forceinline__ void sum_diff(const A2& ab, V& s, V& d)
+    {
+        const ffacc a{f2_x(ab.s), f2_x(ab.c)}, b{f2_y(ab.s), f2_y(ab.c)};
+        if constexpr (LOOSE) {
+            if constexpr (SIGN > 0) acc_sum_diff_loose(b, a, s, d);
+            else acc_sum_diff_loose(a, b, s, d);
+        } else {
+            if constexpr (SIGN > 0) acc_sum_diff(b, a, s, d);
+            else acc_sum_diff(a, b, s, d);
+        }
     }
     static C coef(double d)
     {
@@ -112,14 +178,23 @@ struct EngF32 {
     __device__ static __forceinline__ V mul(V a, V b) { return a * b; }
     __device__ static __forceinline__ V vadd(V a, V b) { return a + b; }
     __device__ static __forceinline__ V vsub(V a, V b) { return a - b; }
-    __device__ static __forceinline__ V vadd_in(V a, V b) { return a + b; }
-    __device__ static __forceinline__ V vsub_in(V a, V b) { return a - b; }
-    __device__ static __forceinline__ void sum_diff(const A& a, const A& b, V& s, V& d)
+    using V2 = f2;
+    using A2 = f2;
+    __device__ static __forceinline__ V2 even_odd(V a, V b) { return f2_make(a + b, a - b); }
+    __device__ static __forceinline__ V even(V2 v) { return f2_x(v); }
+    __device__ static __forceinline__ V odd(V2 v) { return f2_y(v); }
+    __device__ static __forceinline__ A2 first2(const CoefPair<C>& c, V2 v) { return f2_mul(c.v, v); }
+    __device__ static __forceinline__ void madd2(A2& acc, const CoefPair<C>& c, V2 v) { acc = f2_fma(c.v, v, acc); }
+    __device__ static __forceinline__ void madd_even(A2& acc, C c, V x)
     {
-        s = a + b;
-        d = b - a;
+        acc = f2_make(fmaf(c, x, f2_x(acc)), f2_y(acc));
     }
-    __device__ static __forceinline__ void sum_diff_loose(const A& a, const A& b, V& s, V& d) { sum_diff(a, b, s, d); }
+    template <int SIGN, bool LOOSE>
+    __device__ static __forceinline__ void sum_diff(A2 a, V& s, V& d)
+    {
+        s = f2_x(a) + f2_y(a);
+        d = SIGN > 0 ? f2_x(a) - f2_y(a) : f2_y(a) - f2_x(a);
+    }
     static C coef(double d) { return static_cast<float>(d); }
 };
 

@@ -29,6 +29,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cstring>
 
 namespace bkg {
 
@@ -194,6 +195,132 @@ __device__ __forceinline__ ff ff_add(const ff a, const ff b)
     ff r;
     fast_two_sum(s, e, r.hi, r.lo);
     return r;
+}
+
+// ---- packed FP32: two lanes per instruction -----------------------------------
+//
+// add/sub/mul/fma.rn.f32x2 do two IEEE single-precision operations in one
+// issue slot.  Measured on GB300 (cycles per warp instruction and SM
+// sub-partition, 8 warps resident): scalar FADD or FFMA 1.19, packed 2.0 for
+// the two lanes, constant-bank operands included.  The FP32 pipe's rate is
+// the same; the issue slots, which bound the float-float kernels, halve.
+// Each lane is the scalar operation with the same rounding, so packed results
+// are bitwise those of the scalar code.
+typedef unsigned long long f2;   // lane x in the low word, lane y in the high word
+
+__host__ __device__ __forceinline__ f2 f2_make(float x, float y)
+{
+#ifdef __CUDA_ARCH__
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+#else
+    const float t[2] = {x, y};
+    f2 r;
+    memcpy(&r, t, sizeof r);
+    return r;
+#endif
+}
+__device__ __forceinline__ float f2_x(f2 a)
+{
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+    return x;
+}
+__device__ __forceinline__ float f2_y(f2 a)
+{
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+    return y;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b)
+{
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_sub(f2 a, f2 b)
+{
+    f2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b)
+{
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c)
+{
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// a * b rounded, safe next to f2_add / f2_sub: ptxas fuses a packed multiply
+// (and a packed fma with a literal zero) into a following packed add, .rn or
+// not, which would break TwoSum (measured: 40 % of random a - b c differ from
+// the two-step result, -fmad=false included).  The addend -0 comes from
+// constant memory, which the compiler cannot see through; it leaves the
+// rounded product, sign of zero included, unchanged.
+static __constant__ f2 kOpaqueNegZero = 0x8000000080000000ull;
+__device__ __forceinline__ f2 f2_mul_rounded(f2 a, f2 b) { return f2_fma(a, b, kOpaqueNegZero); }
+
+// Two float-float values, one per lane.
+struct ffp {
+    f2 hi;
+    f2 lo;
+};
+__device__ __forceinline__ ffp ffp_make(const ff a, const ff b) { return ffp{f2_make(a.hi, b.hi), f2_make(a.lo, b.lo)}; }
+__device__ __forceinline__ ff ffp_x(const ffp a) { return ff{f2_x(a.hi), f2_x(a.lo)}; }
+__device__ __forceinline__ ff ffp_y(const ffp a) { return ff{f2_y(a.hi), f2_y(a.lo)}; }
+
+// Two coefficients; the hi parts also negated (nhi), because the exact error
+// of a product needs -(a x) and the packed fma has no operand signs.
+struct ffcp {
+    f2 hi;
+    f2 nhi;
+    f2 lo;
+};
+
+// Two compensated accumulators (ffacc), one per lane.
+struct ffaccp {
+    f2 s;
+    f2 c;
+};
+
+// TwoSum in both lanes.
+__device__ __forceinline__ void two_sum2(f2 a, f2 b, f2& s, f2& e)
+{
+    s = f2_add(a, b);
+    const f2 bb = f2_sub(s, a);
+    e = f2_add(f2_sub(a, f2_sub(s, bb)), f2_sub(b, bb));
+}
+
+// The accumulators holding a * x alone (acc_first).
+__device__ __forceinline__ ffaccp acc_first2(const ffcp& a, const ffp x)
+{
+    f2 pe = f2_fma(a.hi, x.hi, f2_mul_rounded(a.nhi, x.hi));
+    pe = f2_fma(a.hi, x.lo, pe);
+    pe = f2_fma(a.lo, x.hi, pe);
+    return ffaccp{f2_mul_rounded(a.hi, x.hi), pe};
+}
+
+// acc += a * x in both lanes (acc_madd): the product is formed negated (np),
+// its exact error is fma(a, x, np), and TwoSum runs on s - np = s + p.
+__device__ __forceinline__ void acc_madd2(ffaccp& acc, const ffcp& a, const ffp x)
+{
+    const f2 np = f2_mul_rounded(a.nhi, x.hi);
+    f2 pe = f2_fma(a.hi, x.hi, np);
+    pe = f2_fma(a.hi, x.lo, pe);
+    pe = f2_fma(a.lo, x.hi, pe);
+    const f2 s = f2_sub(acc.s, np);
+    const f2 bb = f2_sub(s, acc.s);
+    // e = (acc.s - (s - bb)) + (p - bb) = (acc.s - (s - bb)) - (np + bb)
+    const f2 e = f2_sub(f2_sub(acc.s, f2_sub(s, bb)), f2_add(np, bb));
+    acc.s = s;
+    acc.c = f2_add(acc.c, f2_add(e, pe));
 }
 
 // ---- binary64 <-> float-float ------------------------------------------------

@@ -331,8 +331,7 @@ __device__ __forceinline__ void sweep(const typename Eng::V* in, typename Eng::V
 template <class C, int Q>
 struct EOMat {
     static constexpr int H = Q / 2;
-    C A[H * H];
-    C B[H * H];
+    CoefPair<C> AB[H * H];   // (A, B)(o, n)
     C c[H];
     C r[H];
 };
@@ -353,8 +352,7 @@ inline bool make_eo(const double* m, bool trans, EOMat<C, Q>& out, Conv conv)
         }
     for (int o = 0; o < H; ++o) {
         for (int n = 0; n < H; ++n) {
-            out.A[o * H + n] = conv(0.5 * (M(o, n) + M(o, Q - 1 - n)));
-            out.B[o * H + n] = conv(0.5 * (M(o, n) - M(o, Q - 1 - n)));
+            out.AB[o * H + n].set(conv(0.5 * (M(o, n) + M(o, Q - 1 - n))), conv(0.5 * (M(o, n) - M(o, Q - 1 - n))));
         }
         out.c[o] = conv((Q & 1) ? M(o, H) : 0.0);
         out.r[o] = conv((Q & 1) ? M(H, o) : 0.0);
@@ -372,33 +370,25 @@ inline bool make_eo(const double* m, bool trans, EOMat<C, Q>& out, Conv conv)
 template <class Eng, int Q, bool LOOSE = false, class EM>
 __device__ __forceinline__ void eo_line(const typename Eng::V (&x)[Q], typename Eng::V (&y)[Q], const EM& m)
 {
-    using V = typename Eng::V;
     using A = typename Eng::A;
+    using V2 = typename Eng::V2;
+    using A2 = typename Eng::A2;
     constexpr int H = Q / 2;
-    V ev[H > 0 ? H : 1], dv[H > 0 ? H : 1];
+    V2 w[H > 0 ? H : 1];   // (even, odd) combinations
 #pragma unroll
-    for (int n = 0; n < H; ++n) {
-        ev[n] = Eng::vadd_in(x[n], x[Q - 1 - n]);
-        dv[n] = Eng::vsub_in(x[n], x[Q - 1 - n]);
-    }
+    for (int n = 0; n < H; ++n) w[n] = Eng::even_odd(x[n], x[Q - 1 - n]);
 #pragma unroll
     for (int o = 0; o < H; ++o) {
-        A aa = Eng::first(m.A[o * H], ev[0]), bb = Eng::first(m.B[o * H], dv[0]);
+        A2 ab = Eng::first2(m.AB[o * H], w[0]);
 #pragma unroll
-        for (int n = 1; n < H; ++n) {
-            Eng::madd(aa, m.A[o * H + n], ev[n]);
-            Eng::madd(bb, m.B[o * H + n], dv[n]);
-        }
-        if (Q & 1) Eng::madd(aa, m.c[o], x[H]);
-        if constexpr (LOOSE)
-            Eng::sum_diff_loose(aa, bb, y[o], y[Q - 1 - o]);   // a + b, b - a
-        else
-            Eng::sum_diff(aa, bb, y[o], y[Q - 1 - o]);
+        for (int n = 1; n < H; ++n) Eng::madd2(ab, m.AB[o * H + n], w[n]);
+        if (Q & 1) Eng::madd_even(ab, m.c[o], x[H]);
+        Eng::template sum_diff<-1, LOOSE>(ab, y[o], y[Q - 1 - o]);   // a + b, b - a
     }
     if constexpr ((Q & 1) != 0) {
-        A t = Eng::first(m.r[0], dv[0]);
+        A t = Eng::first(m.r[0], Eng::odd(w[0]));
 #pragma unroll
-        for (int n = 1; n < H; ++n) Eng::madd(t, m.r[n], dv[n]);
+        for (int n = 1; n < H; ++n) Eng::madd(t, m.r[n], Eng::odd(w[n]));
         y[H] = LOOSE ? Eng::loose(t) : Eng::result(t);
     }
 }
@@ -438,6 +428,8 @@ __device__ __forceinline__ void sweep_eo_dyn(const typename Eng::V* in, typename
 {
     using V = typename Eng::V;
     using A = typename Eng::A;
+    using V2 = typename Eng::V2;
+    using A2 = typename Eng::A2;
     constexpr int H = Q / 2;
     constexpr int L = Q * Q;
     static_assert(WB::X == 0, "unswizzled boxes");
@@ -454,33 +446,24 @@ __device__ __forceinline__ void sweep_eo_dyn(const typename Eng::V* in, typename
         V x[Q];
 #pragma unroll
         for (int n = 0; n < Q; ++n) x[n] = pi[n * SD];
-        V ev[H > 0 ? H : 1], dv[H > 0 ? H : 1];
+        V2 lw[H > 0 ? H : 1];   // (even, odd) combinations
 #pragma unroll
-        for (int n = 0; n < H; ++n) {
-            ev[n] = Eng::vadd_in(x[n], x[Q - 1 - n]);
-            dv[n] = Eng::vsub_in(x[n], x[Q - 1 - n]);
-        }
+        for (int n = 0; n < H; ++n) lw[n] = Eng::even_odd(x[n], x[Q - 1 - n]);
 #pragma unroll
         for (int o = 0; o < H; ++o) {
-            A aa = Eng::first(m.A[o * H], ev[0]), bb = Eng::first(m.B[o * H], dv[0]);
+            A2 ab = Eng::first2(m.AB[o * H], lw[0]);
 #pragma unroll
-            for (int n = 1; n < H; ++n) {
-                Eng::madd(aa, m.A[o * H + n], ev[n]);
-                Eng::madd(bb, m.B[o * H + n], dv[n]);
-            }
-            if (Q & 1) Eng::madd(aa, m.c[o], x[H]);
+            for (int n = 1; n < H; ++n) Eng::madd2(ab, m.AB[o * H + n], lw[n]);
+            if (Q & 1) Eng::madd_even(ab, m.c[o], x[H]);
             V s, d;
-            if constexpr (LOOSE)
-                Eng::sum_diff_loose(aa, bb, s, d);   // a + b, b - a
-            else
-                Eng::sum_diff(aa, bb, s, d);
+            Eng::template sum_diff<-1, LOOSE>(ab, s, d);   // a + b, b - a
             po[o * SD] = s;
             po[(Q - 1 - o) * SD] = d;
         }
         if (Q & 1) {
-            A t = Eng::first(m.r[0], dv[0]);
+            A t = Eng::first(m.r[0], Eng::odd(lw[0]));
 #pragma unroll
-            for (int n = 1; n < H; ++n) Eng::madd(t, m.r[n], dv[n]);
+            for (int n = 1; n < H; ++n) Eng::madd(t, m.r[n], Eng::odd(lw[n]));
             po[H * SD] = Eng::result(t);
         }
     }
@@ -498,8 +481,7 @@ template <class C, int NO, int NI>
 struct EORMat {
     static constexpr int HO = NO / 2;
     static constexpr int HI = NI / 2;
-    C A[HO * HI > 0 ? HO * HI : 1];
-    C B[HO * HI > 0 ? HO * HI : 1];
+    CoefPair<C> AB[HO * HI > 0 ? HO * HI : 1];   // (A, B)(o, n)
     C c[HO > 0 ? HO : 1];
     C r[HI > 0 ? HI : 1];
     C rm;
@@ -523,8 +505,7 @@ inline bool make_eor(const double* m, int ld, bool trans, int sign, EORMat<C, NO
         }
     for (int o = 0; o < HO; ++o) {
         for (int n = 0; n < HI; ++n) {
-            out.A[o * HI + n] = conv(0.5 * (M(o, n) + M(o, NI - 1 - n)));
-            out.B[o * HI + n] = conv(0.5 * (M(o, n) - M(o, NI - 1 - n)));
+            out.AB[o * HI + n].set(conv(0.5 * (M(o, n) + M(o, NI - 1 - n))), conv(0.5 * (M(o, n) - M(o, NI - 1 - n))));
         }
         out.c[o] = conv((NI & 1) ? M(o, HI) : 0.0);
     }
@@ -539,40 +520,28 @@ inline bool make_eor(const double* m, int ld, bool trans, int sign, EORMat<C, NO
 template <class Eng, int NI, int NO, int SIGN, bool LOOSE = false, class EM>
 __device__ __forceinline__ void eor_line(const typename Eng::V (&x)[NI], typename Eng::V (&y)[NO], const EM& m)
 {
-    using V = typename Eng::V;
     using A = typename Eng::A;
+    using V2 = typename Eng::V2;
+    using A2 = typename Eng::A2;
     constexpr int HI = NI / 2, HO = NO / 2;
-    V ev[HI > 0 ? HI : 1], dv[HI > 0 ? HI : 1];
+    V2 w[HI > 0 ? HI : 1];   // (even, odd) combinations
 #pragma unroll
-    for (int n = 0; n < HI; ++n) {
-        ev[n] = Eng::vadd_in(x[n], x[NI - 1 - n]);
-        dv[n] = Eng::vsub_in(x[n], x[NI - 1 - n]);
-    }
+    for (int n = 0; n < HI; ++n) w[n] = Eng::even_odd(x[n], x[NI - 1 - n]);
+    auto mid = [&](int n) { return SIGN > 0 ? Eng::even(w[n]) : Eng::odd(w[n]); };
     if constexpr ((NO & 1) != 0) {
-        A t = Eng::first(m.r[0], SIGN > 0 ? ev[0] : dv[0]);
+        A t = Eng::first(m.r[0], mid(0));
 #pragma unroll
-        for (int n = 1; n < HI; ++n) Eng::madd(t, m.r[n], SIGN > 0 ? ev[n] : dv[n]);
+        for (int n = 1; n < HI; ++n) Eng::madd(t, m.r[n], mid(n));
         if constexpr (SIGN > 0 && (NI & 1) != 0) Eng::madd(t, m.rm, x[HI]);
         y[HO] = LOOSE ? Eng::loose(t) : Eng::result(t);
     }
 #pragma unroll
     for (int o = 0; o < HO; ++o) {
-        A aa = Eng::first(m.A[o * HI], ev[0]), bb = Eng::first(m.B[o * HI], dv[0]);
+        A2 ab = Eng::first2(m.AB[o * HI], w[0]);
 #pragma unroll
-        for (int n = 1; n < HI; ++n) {
-            Eng::madd(aa, m.A[o * HI + n], ev[n]);
-            Eng::madd(bb, m.B[o * HI + n], dv[n]);
-        }
-        if constexpr ((NI & 1) != 0) Eng::madd(aa, m.c[o], x[HI]);
-        if constexpr (SIGN > 0 && LOOSE) {
-            Eng::sum_diff_loose(bb, aa, y[o], y[NO - 1 - o]);   // b + a, a - b
-        } else if constexpr (SIGN > 0) {
-            Eng::sum_diff(bb, aa, y[o], y[NO - 1 - o]);
-        } else if constexpr (LOOSE) {
-            Eng::sum_diff_loose(aa, bb, y[o], y[NO - 1 - o]);   // a + b, b - a
-        } else {
-            Eng::sum_diff(aa, bb, y[o], y[NO - 1 - o]);
-        }
+        for (int n = 1; n < HI; ++n) Eng::madd2(ab, m.AB[o * HI + n], w[n]);
+        if constexpr ((NI & 1) != 0) Eng::madd_even(ab, m.c[o], x[HI]);
+        Eng::template sum_diff<SIGN, LOOSE>(ab, y[o], y[NO - 1 - o]);   // a + b, SIGN (a - b)
     }
 }
 
