@@ -19,9 +19,9 @@ namespace bkg {
 
 // The even and the odd half of a line's contraction (EOMat, EORMat) run side
 // by side, one per lane: a coefficient pair C2 (even lane, odd lane), a value
-// pair V2 and an accumulator pair A2 per engine.  FP32-pipe engines hold them
-// packed (two lanes per instruction, bk_ff.cuh), the DFMA engine as two
-// doubles.
+// pair V2 and an accumulator pair A2 per engine.  The FP32-pipe engines use
+// packed operations (two lanes per instruction, bk_ff.cuh), the DFMA engine
+// two doubles.
 template <class C>
 struct CoefPair;
 template <>
@@ -42,9 +42,8 @@ template <>
 struct CoefPair<ff> : ffcp {
     void set(ff a, ff b)
     {
-        hi = f2_make(a.hi, b.hi);
-        nhi = f2_make(-a.hi, -b.hi);
-        lo = f2_make(a.lo, b.lo);
+        x = a;
+        y = b;
     }
 };
 
@@ -55,7 +54,14 @@ struct EngDfma {
     using A = double;
     static constexpr int kId = BK_ENGINE_DFMA;
     __device__ static __forceinline__ V load(S x) { return x; }
+    template <int N>
+    __device__ static __forceinline__ void load_n(const S (&x)[N], V (&y)[N])
+    {
+#pragma unroll
+        for (int i = 0; i < N; ++i) y[i] = x[i];
+    }
     __device__ static __forceinline__ S store(V x) { return x; }
+    __device__ static __forceinline__ S store(V x, bool) { return x; }
     __device__ static __forceinline__ A zero() { return 0.0; }
     // an accumulator started with a first product / value (no add to zero)
     __device__ static __forceinline__ A first(C c, V x) { return c * x; }
@@ -104,7 +110,20 @@ struct EngFF {
     __device__ static __forceinline__ V load(S x) { return split(x); }
     // a value split ahead of time (bk_g_to_ff): no work
     __device__ static __forceinline__ V load(ff2 x) { return ff{x.hi, x.lo}; }
+    template <int N>
+    __device__ static __forceinline__ void load_n(const S (&x)[N], V (&y)[N])
+    {
+        split_n(x, y);
+    }
+    template <int N>
+    __device__ static __forceinline__ void load_n(const ff2 (&x)[N], V (&y)[N])
+    {
+#pragma unroll
+        for (int i = 0; i < N; ++i) y[i] = load(x[i]);
+    }
     __device__ static __forceinline__ S store(V x) { return join(x); }
+    // fp64: on the FP64 pipe
+    __device__ static __forceinline__ S store(V x, bool fp64) { return fp64 ? join_fp64(x) : join(x); }
     __device__ static __forceinline__ A zero() { return acc_zero(); }
     // the first product needs no TwoSum into an empty accumulator
     __device__ static __forceinline__ A first(C c, V x) { return acc_first(c, x); }
@@ -124,10 +143,10 @@ struct EngFF {
     // operands of multiply-adds only: not renormalised
     __device__ static __forceinline__ V2 even_odd(V a, V b)
     {
-        return ffp_make(ff_add_loose(a, b), ff_add_loose(a, ff{-b.hi, -b.lo}));
+        return ffp{ff_add_loose(a, b), ff_add_loose(a, ff{-b.hi, -b.lo})};
     }
-    __device__ static __forceinline__ V even(const V2& v) { return ffp_x(v); }
-    __device__ static __forceinline__ V odd(const V2& v) { return ffp_y(v); }
+    __device__ static __forceinline__ V even(const V2& v) { return v.x; }
+    __device__ static __forceinline__ V odd(const V2& v) { return v.y; }
     __device__ static __forceinline__ A2 first2(const CoefPair<C>& c, const V2& v) { return acc_first2(c, v); }
     __device__ static __forceinline__ void madd2(A2& acc, const CoefPair<C>& c, const V2& v) { acc_madd2(acc, c, v); }
     __device__ static __forceinline__ void madd_even(A2& acc, C c, V x)
@@ -165,7 +184,14 @@ struct EngF32 {
     using A = float;
     static constexpr int kId = 100;
     __device__ static __forceinline__ V load(S x) { return x; }
+    template <int N>
+    __device__ static __forceinline__ void load_n(const S (&x)[N], V (&y)[N])
+    {
+#pragma unroll
+        for (int i = 0; i < N; ++i) y[i] = x[i];
+    }
     __device__ static __forceinline__ S store(V x) { return x; }
+    __device__ static __forceinline__ S store(V x, bool) { return x; }
     __device__ static __forceinline__ A zero() { return 0.0f; }
     __device__ static __forceinline__ A first(C c, V x) { return c * x; }
     __device__ static __forceinline__ A vfirst(V a, V x) { return a * x; }

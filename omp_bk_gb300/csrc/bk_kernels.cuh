@@ -693,8 +693,8 @@ __device__ __forceinline__ void ilines(int ne, int tid, int nt, F f)
     }
 }
 
-// The points n0, n0 + NS, n0 + 2 NS, ... (< Q) of one line, f(n) for each:
-// NS = 1 walks the whole line at compile-time n; with NS > 1 (a line split
+// The points n0, n0 + NS, n0 + 2 NS, ... (< Q) of one line, f(n, m) for the
+// m-th of them (m a compile-time constant): NS = 1 walks the whole line at compile-time n; with NS > 1 (a line split
 // among NS thread groups, n0 the group) the offsets n * stride are the
 // per-line n0 * stride plus compile-time multiples.
 template <int Q, int NS, class F>
@@ -703,20 +703,22 @@ __device__ __forceinline__ void line_points(const int n0, F f)
 #pragma unroll
     for (int m = 0; m < (Q + NS - 1) / NS; ++m) {
         if (NS == 1) {
-            f(m);
+            f(m, m);
         } else {
             const int n = n0 + m * NS;
-            if (n < Q) f(n);
+            if (n < Q) f(n, m);
         }
     }
 }
 
-// Padded work box -> dense (X, Y, Z) S values.
+// Padded work box -> dense (X, Y, Z) S values, every other one of a thread
+// converted on the FP64 pipe (Eng::store).
 template <class Eng, class WB, int X, int Y, int Z>
 __device__ __forceinline__ void store_box(const typename Eng::V* src, typename Eng::S* dst, int estride, int ne,
                                           int tid, int nt)
 {
     constexpr int N = X * Y * Z;
+    bool alt = true;
     for (int w = tid; w < ne * N; w += nt) {
         const int e = w / N;
         const int x = w - e * N;
@@ -724,7 +726,8 @@ __device__ __forceinline__ void store_box(const typename Eng::V* src, typename E
         const int r = x - i * (Y * Z);
         const int j = r / Z;
         const int k = r - j * Z;
-        dst[e * estride + x] = Eng::store(src[e * WB::size + WB::at(i, j, k)]);
+        dst[e * estride + x] = Eng::store(src[e * WB::size + WB::at(i, j, k)], alt);
+        alt = !alt;
     }
 }
 
@@ -778,6 +781,25 @@ inline bool make_p13_eo(P13<C, Q>& p, const double* B, const double* D, Conv con
     return ok;
 }
 
+// ---- fluxes --------------------------------------------------------------------
+
+// The fluxes G grad u at one point (symmetric factors g rr rs rt ss st tt for
+// F = 6, the full 3 x 3 tensor row-major for F = 9) from the gradient q.
+template <class Eng, int F>
+__device__ __forceinline__ void point_flux(const typename Eng::V (&g)[F], const typename Eng::V (&q)[3],
+                                           typename Eng::V (&r)[3])
+{
+    constexpr int sym[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        auto gi = [&](int b) { return F == 6 ? g[sym[a][b]] : g[3 * a + b]; };
+        typename Eng::A acc = Eng::vfirst(gi(0), q[0]);
+        Eng::vmadd(acc, gi(1), q[1]);
+        Eng::vmadd(acc, gi(2), q[2]);
+        r[a] = Eng::result(acc);
+    }
+}
+
 // ---- BK5 -----------------------------------------------------------------------
 
 // Index of factor f at point (i, j, k) within an element's G.
@@ -805,6 +827,12 @@ struct BK5Cfg {
     static constexpr int STAGE_BYTES = U_BYTES + G_BYTES;
     static constexpr int W_BYTES = ((NBOX * EB * WB::size * int(sizeof(V)) + 15) / 16) * 16;
     static constexpr int SMEM = STAGE_BYTES + W_BYTES + 16;
+    // resident blocks asked of the register allocator (DPAR): what shared
+    // memory allows (1 KB per block is the system's), down to 56 registers a
+    // thread; the flux pass would take up to 107 and halve the blocks
+    static constexpr int BY_SMEM = 233472 / (SMEM + 1024) < 1 ? 1 : 233472 / (SMEM + 1024);
+    static constexpr int BY_REGS = 65536 / (NT * 56) < 1 ? 1 : 65536 / (NT * 56);
+    static constexpr int MINB = DPAR == 0 ? 1 : (BY_SMEM < BY_REGS ? BY_SMEM : BY_REGS);
 };
 
 // One batch of ne elements of order Q whose u (us, dense; shared or global
@@ -881,6 +909,10 @@ __device__ __forceinline__ void bk5_sweep_batch(const typename Eng::C* __restric
     // those blocks walk the points flat (point w of the batch, its indices
     // by division), which spreads them evenly over all threads.
     constexpr bool FLAT = DPAR != 0 && Q % 3 == 1;
+    // float-float: part of the joins on the FP64 pipe (join_fp64), every other
+    // point (all where the walk is flat).  Not at Q = 9, whose one block per
+    // SM runs the last pass alone (981 -> 1036 us)
+    constexpr bool JOIN64 = !(DPAR != 0 && Q >= 9);
     constexpr int LS = DPAR ? 3 : 1;
     const int lt = DPAR ? tg : tid;     // the thread's first line
     const int lnt = DPAR ? ntd : nt;    // threads per line set
@@ -891,7 +923,7 @@ __device__ __forceinline__ void bk5_sweep_batch(const typename Eng::C* __restric
         load_box<Eng, WB, Q, Q, Q>(us, Q3, W2, ne, tid, nt);
     } else if (lact) {
         ilines<WB, Q, Q, Q>(ne, lt, lnt, [&](int, int, int, int d, int b) {
-            line_points<Q, LS>(ln0, [&](int i) { W2[b + i * WB::PS] = Eng::load(us[d + i * Q * Q]); });
+            line_points<Q, LS>(ln0, [&](int i, int) { W2[b + i * WB::PS] = Eng::load(us[d + i * Q * Q]); });
         });
     }
     __syncthreads();
@@ -915,67 +947,57 @@ __device__ __forceinline__ void bk5_sweep_batch(const typename Eng::C* __restric
         sweep<Eng, WB, 2, Q, Q, Q, Q>(W2, W2, ne, Dm, tid, nt);
     }
     __syncthreads();
-    // 4. fluxes with the symmetric (F = 6) or full (F = 9) factors
-    //    (point wi of the boxes, g(f) the point's factor f)
-    auto flux = [&](const int wi, auto g) {
-        const V qr = W0[wi], qs = W1[wi], qt = QT[wi];
-        A r0, r1, r2;
-        if (F == 6) {
-            const V g0 = g(0), g1 = g(1), g2 = g(2), g3 = g(3), g4 = g(4), g5 = g(5);
-            r0 = Eng::vfirst(g0, qr); Eng::vmadd(r0, g1, qs); Eng::vmadd(r0, g2, qt);
-            r1 = Eng::vfirst(g1, qr); Eng::vmadd(r1, g3, qs); Eng::vmadd(r1, g4, qt);
-            r2 = Eng::vfirst(g2, qr); Eng::vmadd(r2, g4, qs); Eng::vmadd(r2, g5, qt);
-        } else {
-            r0 = Eng::vfirst(g(0), qr); Eng::vmadd(r0, g(1), qs); Eng::vmadd(r0, g(2), qt);
-            r1 = Eng::vfirst(g(3), qr); Eng::vmadd(r1, g(4), qs); Eng::vmadd(r1, g(5), qt);
-            r2 = Eng::vfirst(g(6), qr); Eng::vmadd(r2, g(7), qs); Eng::vmadd(r2, g(8), qt);
+    // 4. fluxes with the symmetric (F = 6) or full (F = 9) factors at point n
+    //    of line r: lines (i, j) along k with G in the column layout (G(e, f,
+    //    k, i, j) of consecutive lines is consecutive), lines (j, k) along i
+    //    otherwise
+    auto flux = [&](const int e, const int r, const int n) {
+        const int a = r / Q, b = r - a * Q;
+        const int w = e * WB::size + (LAYOUT == 2 ? WB::at(a, b, n) : WB::at(n, a, b));
+        const GS* ge = gs + e * F * Q3 + (LAYOUT == 2 ? n * (Q * Q) + r : g_index<Eng, Q, F, LAYOUT>(n, a, 0, b));
+        constexpr int FS = LAYOUT == 1 ? Q : Q3;   // stride of the factors
+        V g[F], fl[3];
+        // one range test and branch per GN factors: all of them, but at Q = 8
+        // (80 registers) in two halves (735 -> 711 us)
+        constexpr int GN = (Q == 8 && F == 6) ? 3 : F;
+#pragma unroll
+        for (int f0 = 0; f0 < F; f0 += GN) {
+            GS raw[GN];
+            V gv[GN];
+#pragma unroll
+            for (int f = 0; f < GN; ++f) raw[f] = ge[(f0 + f) * FS];
+            Eng::load_n(raw, gv);
+#pragma unroll
+            for (int f = 0; f < GN; ++f) g[f0 + f] = gv[f];
         }
-        W0[wi] = Eng::result(r0);
-        W1[wi] = Eng::result(r1);
-        QT[wi] = Eng::result(r2);
+        const V q[3] = {W0[w], W1[w], QT[w]};
+        point_flux<Eng, F>(g, q, fl);
+        W0[w] = fl[0];
+        W1[w] = fl[1];
+        QT[w] = fl[2];
     };
-    if constexpr (FLAT) {
-        for (int w = tid; w < ne * Q3; w += nt) {
-            const int e = w / Q3;
-            const int x = w - e * Q3;
-            int i, j, k;
-            if (LAYOUT == 2) {   // walk points in G's (k, i, j) order
-                k = x / (Q * Q);
-                i = (x / Q) % Q;
-                j = x % Q;
-            } else {
-                i = x / (Q * Q);
-                j = (x / Q) % Q;
-                k = x % Q;
-            }
-            const GS* ge = gs + e * F * Q3;
-            flux(e * WB::size + WB::at(i, j, k),
-                 [&](int f) { return Eng::load(ge[g_index<Eng, Q, F, LAYOUT>(i, j, f, k)]); });
+    if constexpr (DPAR != 0 && Q % 3 == 0) {
+        // a third of each line's points per group (p = 8: 978 -> 958 us against
+        // the walk below)
+        for (int l = tg; l < ne * Q * Q; l += ntd) {
+            const int e = l / (Q * Q);
+            const int r = l - e * (Q * Q);
+            line_points<Q, 3>(grp, [&](int n, int) { flux(e, r, n); });
         }
-    } else if (lact) {
-        if constexpr (LAYOUT == 2) {
-            // lines along k, one per (e, i, j): G(e, f, k, i, j) of
-            // consecutive threads is consecutive
-            for (int l = lt; l < ne * Q * Q; l += lnt) {
-                const int e = l / (Q * Q);
-                const int r = l - e * (Q * Q);   // i*Q + j
-                const int i = r / Q;
-                const int j = r - i * Q;
-                const int wb = e * WB::size + WB::at(i, j, 0);
-                const GS* ge = gs + e * F * Q3 + r;
-                line_points<Q, LS>(ln0, [&](int k) {
-                    flux(wb + k, [&](int f) { return Eng::load(ge[(f * Q + k) * Q * Q]); });
-                });
-            }
-        } else {
-            // lines along i, one per (e, j, k)
-            ilines<WB, Q, Q, Q>(ne, lt, lnt, [&](int e, int j, int k, int, int b) {
-                const GS* ge = gs + e * F * Q3;
-                line_points<Q, LS>(ln0, [&](int i) {
-                    flux(b + i * WB::PS,
-                         [&](int f) { return Eng::load(ge[g_index<Eng, Q, F, LAYOUT>(i, j, f, k)]); });
-                });
-            });
+    } else if constexpr (DPAR != 0) {
+        // Q not a multiple of three: the points of all lines over all threads,
+        // consecutive threads on consecutive lines
+        for (int w = tid; w < ne * Q3; w += nt) {
+            const int t = w / (Q * Q);
+            const int e = t / Q;
+            flux(e, w - t * (Q * Q), t - e * Q);
+        }
+    } else {
+        for (int l = tid; l < ne * Q * Q; l += nt) {
+            const int e = l / (Q * Q);
+            const int r = l - e * (Q * Q);
+#pragma unroll
+            for (int n = 0; n < Q; ++n) flux(e, r, n);
         }
     }
     __syncthreads();
@@ -1041,7 +1063,8 @@ __device__ __forceinline__ void bk5_sweep_batch(const typename Eng::C* __restric
     //    arithmetic (double for the FP64 engines).  The loop is written twice
     //    (with and without the mass term) so that no point carries the
     //    predicated-off mass arithmetic.
-    auto last_point = [&](auto with_mass, const int w, const int wi) {
+    //    alt: the value joined on the FP64 pipe (JOIN64)
+    auto last_point = [&](auto with_mass, const int w, const int wi, const bool alt) {
         V res;
         if constexpr (EO) {
             if constexpr (HasSum3<Eng>::value) {
@@ -1055,7 +1078,7 @@ __device__ __forceinline__ void bk5_sweep_batch(const typename Eng::C* __restric
         } else {
             res = W2[wi];
         }
-        S out = Eng::store(res);
+        S out = Eng::store(res, JOIN64 && alt);
         if constexpr (decltype(with_mass)::value) out += lam * mb[w] * us[w];
         vb[w] = out;
         if constexpr (DOT) acc_madd_f(*dot, us[w], out);   // u . A u for CG, compensated
@@ -1068,11 +1091,13 @@ __device__ __forceinline__ void bk5_sweep_batch(const typename Eng::C* __restric
                 const int i = x / (Q * Q);
                 const int j = (x / Q) % Q;
                 const int k = x % Q;
-                last_point(with_mass, w, e * WB::size + WB::at(i, j, k));
+                last_point(with_mass, w, e * WB::size + WB::at(i, j, k), true);
             }
         } else if (lact) {
             ilines<WB, Q, Q, Q>(ne, lt, lnt, [&](int, int, int, int d, int b) {
-                line_points<Q, LS>(ln0, [&](int i) { last_point(with_mass, d + i * Q * Q, b + i * WB::PS); });
+                line_points<Q, LS>(ln0, [&](int i, int m) {
+                    last_point(with_mass, d + i * Q * Q, b + i * WB::PS, m % 2 == 0);
+                });
             });
         }
     };
@@ -1095,7 +1120,7 @@ __device__ __forceinline__ void bk5_sweep_batch(const typename Eng::C* __restric
                     Eng::add(acc, W1[la(o)]);
                     res = Eng::loose(acc);   // store() renormalises
                 }
-                S out = Eng::store(res);
+                S out = Eng::store(res, JOIN64 && o % 2 == 0);
                 if constexpr (decltype(with_mass)::value) out += lam * mb[w0 + o] * us[w0 + o];
                 vb[w0 + o] = out;
                 if constexpr (DOT) acc_madd_f(*dot, us[w0 + o], out);
@@ -1124,7 +1149,7 @@ __device__ __forceinline__ void bk5_sweep_batch(const typename Eng::C* __restric
 // mass term reads it there), so the copies overlap the transposed sweeps and
 // the last pass instead of stalling the block at the start of each batch.
 template <class Eng, int Q, int EB, int F, int LAYOUT, bool EO = false, int DPAR = 0, class GS = typename Eng::S>
-__global__ void __launch_bounds__(BK5Cfg<Eng, Q, EB, F, LAYOUT, DPAR>::NT)
+__global__ void __launch_bounds__(BK5Cfg<Eng, Q, EB, F, LAYOUT, DPAR>::NT, BK5Cfg<Eng, Q, EB, F, LAYOUT, DPAR>::MINB)
     bk5_kernel(const __grid_constant__ P5<typename Eng::C, Q> prm, const long long E,
                const typename Eng::S* __restrict__ u, const GS* __restrict__ G,
                const typename Eng::S* __restrict__ mass, const double lambda, typename Eng::S* __restrict__ v,
@@ -1444,23 +1469,22 @@ __global__ void __launch_bounds__(BK3Cfg<Eng, Q, EB, DPAR>::NT)
                 const int x = w - e * Q3;
                 const int i = x / (Q * Q), j = (x / Q) % Q, k = x % Q;
                 const int wi = e * WB::size + WB::at(i, j, k);
-                V qr = W0[wi], qs = W1[wi], qt = W3[wi];
+                V q[3] = {W0[wi], W1[wi], W3[wi]};
                 if constexpr (decltype(with_k)::value) {
                     const V kk = Eng::load(ks[e * Q3 + x]);
-                    qr = Eng::mul(kk, qr);
-                    qs = Eng::mul(kk, qs);
-                    qt = Eng::mul(kk, qt);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) q[c] = Eng::mul(kk, q[c]);
                 }
                 const GS* ge = gs + e * 6 * Q3 + x;   // factor-major
-                const V g0 = Eng::load(ge[0]), g1 = Eng::load(ge[Q3]), g2 = Eng::load(ge[2 * Q3]);
-                const V g3 = Eng::load(ge[3 * Q3]), g4 = Eng::load(ge[4 * Q3]), g5 = Eng::load(ge[5 * Q3]);
-                A r0 = Eng::vfirst(g0, qr), r1 = Eng::vfirst(g1, qr), r2 = Eng::vfirst(g2, qr);
-                Eng::vmadd(r0, g1, qs); Eng::vmadd(r0, g2, qt);
-                Eng::vmadd(r1, g3, qs); Eng::vmadd(r1, g4, qt);
-                Eng::vmadd(r2, g4, qs); Eng::vmadd(r2, g5, qt);
-                W0[wi] = Eng::result(r0);
-                W1[wi] = Eng::result(r1);
-                W3[wi] = Eng::result(r2);
+                GS raw[6];
+#pragma unroll
+                for (int f = 0; f < 6; ++f) raw[f] = ge[f * Q3];
+                V g[6], fl[3];
+                Eng::load_n(raw, g);
+                point_flux<Eng, 6>(g, q, fl);
+                W0[wi] = fl[0];
+                W1[wi] = fl[1];
+                W3[wi] = fl[2];
             }
         };
         // the transposed k-direction derivative of the third flux plus the

@@ -473,3 +473,34 @@ def test_bk5_fp64_smooth_field(bklib, p, h):
         bklib.bk5_apply(p, E, D, G, u, v, prec=bklib.PREC_FP64, engine=eng, layout=bklib.LAYOUT_COLUMN)
         torch.cuda.synchronize()
         assert oracle.rel_maxdiff(host(v[: n * Q ** 3]), ref) < TOL64, (eng, p, h)
+
+
+@pytest.mark.parametrize("bk", [3, 5])
+@pytest.mark.parametrize("p", P_ALL)
+def test_fp64_factor_ranges(bklib, bk, p):
+    """The float-float engine splits a point's six factors behind one range
+    test: zeros of both signs and values below the fast range (2^-74) beside
+    ordinary ones take the careful path for the point, at batch remainders of
+    every order's elements per block.  The bound is the FP64 target (the
+    small factors contribute nothing to it: they are below 1e-25)."""
+    E = 29
+    Q, P = (p + 1, p + 1) if bk == 5 else (p + 2, p + 1)
+    rng = np.random.default_rng(100 * bk + p)
+    u = rng.uniform(-1, 1, E * P ** 3)
+    G = rng.uniform(0.1, 1, (E, 6, Q, Q, Q))
+    kind = rng.integers(0, 6, G.shape)
+    G = np.where(kind == 0, 0.0, np.where(kind == 1, -0.0, np.where(kind == 2, G * 1e-26, G)))
+    if bk == 5:
+        D = np.asarray(bklib.bk5_matrices(p)[0])
+        ref = oracle.bk5(Q, E, D, G.transpose(0, 2, 3, 1, 4).copy().ravel(), u)
+        gd, ud = dev(G.transpose(0, 1, 4, 2, 3).copy().ravel(), "f64"), dev(u, "f64")
+        v = torch.full_like(ud, float("nan"))
+        bklib.bk5_apply(p, E, D, gd, ud, v, layout=bklib.LAYOUT_COLUMN)
+    else:
+        B, D = (np.asarray(m) for m in bklib.bk1_bk3_matrices(p)[:2])
+        ref = oracle.bk3(Q, E, B, D, G.ravel(), u)
+        gd, ud = dev(G.ravel(), "f64"), dev(u, "f64")
+        v = torch.full_like(ud, float("nan"))
+        bklib.bk3_apply(p, E, B, D, gd, ud, v)
+    torch.cuda.synchronize()
+    assert oracle.rel_maxdiff(host(v), ref) < TOL64
