@@ -52,31 +52,54 @@ using Eng = EngMixed;
 
 namespace BK_TU_NS {
 
-// Elements per block: about 128 lines per sweep (Q^2 lines per element).
+// Elements per block where no measurement says otherwise: about 128 lines per
+// sweep (Q^2 lines per element).
 constexpr int default_eb(int q) { return (q * q >= 100) ? 1 : ((q * q >= 64) ? 2 : (128 + q * q - 1) / (q * q)); }
 
-// Elements per block of the BK5 and BK3 sweep kernels (even-odd path), the
-// fastest of EB = 1..16 measured per engine and q on GB300 (about 2^24 DoFs
-// per apply).  Small orders want many elements per block (short lines, small
-// boxes); from q = 8 one element per block, whose smaller shared-memory
-// footprint keeps more blocks resident, wins for the FP32-pipe engines.
+// Elements per block of the even-odd kernels, the fastest measured per engine
+// and q on GB300 at 2^23..2^26 points per apply.  A sweep gives each thread a
+// line, so an EB whose EB q^2 lines just fill whole warps leaves no thread
+// idle: q = 3: 7 or 14 (63, 126 lines), q = 5: 5 (125), q = 6: 7 (252),
+// q = 7: 5 (245).  Where fewer elements per block let more blocks share an
+// SM, that wins (from q = 7 the FP32-storage forms, one element).  Times in us
+// (previous choice -> this): float-float BK5 q = 3 262 -> 217, q = 5 716 ->
+// 597, BK3 q = 3 246 -> 221, q = 5 447 -> 399, BK1 q = 3 203 -> 185, q = 9
+// 485 -> 430; FP32 BK5 q = 2 297 -> 250, q = 3 262 -> 244, q = 5 220 -> 197,
+// BK3 q = 6 254 -> 234, q = 7 253 -> 235, BK1 q = 3 216 -> 187, q = 7 178 ->
+// 162, q = 9 170 -> 145.
 constexpr bool eng_is_dfma() { return Eng::kId == BK_ENGINE_DFMA; }
 constexpr bool eng_is_ff() { return Eng::kId == BK_ENGINE_FF; }
 constexpr int sweep_eb5(int q)
 {
-    if (q <= 3) return eng_is_ff() || eng_is_dfma() ? 16 : 12;
-    if (q == 4) return 8;
-    if (eng_is_dfma()) return q == 5 ? 6 : q == 6 ? 4 : q == 7 ? 3 : q == 8 ? 2 : 3;
-    if (eng_is_ff()) return q == 5 ? 4 : q == 6 ? 3 : q == 7 ? 4 : 1;
-    return q == 5 ? 4 : q == 6 ? 3 : q == 7 ? 2 : 1;
+    if (eng_is_dfma()) return q <= 3 ? 16 : q == 4 ? 8 : q == 5 ? 6 : q == 6 ? 4 : q == 7 ? 3 : q == 8 ? 2 : 3;
+    if (q == 2) return 16;
+    if (q == 3) return eng_is_ff() ? 7 : 14;
+    if (q <= 6) return q == 4 ? 8 : q == 5 ? 5 : 3;
+    return eng_is_ff() && q == 7 ? 4 : 1;
 }
 constexpr int sweep_eb3(int q)
 {
-    if (q <= 3) return eng_is_ff() ? 12 : 16;
-    if (q == 4) return 8;
-    if (eng_is_dfma()) return q == 5 ? 6 : q == 6 ? 4 : q == 7 ? 3 : q == 8 ? 2 : q == 9 ? 3 : 1;
-    if (eng_is_ff()) return q == 5 ? 8 : q <= 7 ? 3 : 1;
-    return q == 5 ? 6 : q == 6 ? 4 : q == 7 ? 3 : 1;
+    if (eng_is_dfma())
+        return q <= 3 ? 16 : q == 4 ? 8 : q == 5 ? 6 : q == 6 ? 4 : q == 7 ? 3 : q == 8 ? 2 : q == 9 ? 3 : 1;
+    if (q <= 4) return q == 3 ? 14 : 8;
+    if (eng_is_ff()) return q == 5 ? 10 : q == 6 ? 3 : 1;
+    return q == 5 ? 5 : q == 6 ? 7 : 1;
+}
+// BK1.  At q = 5 the FP32-storage forms also run at EB = 10 (172 -> 166 us at
+// E = 500000); 5 keeps the smaller blocks for the small applies
+constexpr int sweep_eb1(int q)
+{
+    if (eng_is_dfma()) return default_eb(q);
+    if (eng_is_ff()) return q == 3 ? 14 : q == 8 ? 1 : q == 9 ? 3 : default_eb(q);
+    constexpr int t[8] = {14, 8, 5, 7, 5, 1, 1, 1};   // q = 3..10
+    return t[q - 3];
+}
+// the BK3 adjoint (six boxes and two gradients per element)
+constexpr int adj_eb(int q)
+{
+    if (eng_is_dfma()) return default_eb(q) / 2 > 0 ? default_eb(q) / 2 : 1;
+    if (eng_is_ff()) return q == 3 ? 7 : q == 4 ? 4 : q == 5 ? 5 : q == 6 ? 3 : 1;
+    return q == 3 ? 14 : q == 4 ? 8 : q == 5 ? 5 : q == 6 ? 3 : 1;
 }
 
 // Sets the dynamic shared-memory size of a kernel on the current device once
@@ -137,11 +160,13 @@ constexpr int fit_eb5()
 }
 
 // The direction-parallel even-odd shape (three thread groups, one direction
-// each, one shared code body: DPAR = 2) for the float-float engine where it
-// measured faster on GB300: q = 6 (EB 4), 7 (EB 2), 8 (EB 1) and 9 (EB 3),
-// 2-33 % over one thread per line (q = 8: 36.9 against 30.2 GDoF/s).
-constexpr bool sweep_dpar5(int q) { return eng_is_ff() && q >= 6 && q <= 9; }
-constexpr int sweep_eb5_dpar(int q) { return q == 6 ? 4 : q == 7 ? 2 : q == 9 ? 3 : 1; }
+// each) for the float-float engine where it measured faster on GB300: q = 8
+// (EB 1, one code body for the three directions: 711 us against 910 with one
+// thread per line at E = 65536) and q = 9 (EB 3, a body per direction: 939
+// against 1010, one shared body 958, at E = 46000).  q = 6 and 7 run one
+// thread per line (857 against 869, 875 against 899).
+constexpr int sweep_dpar5(int q) { return !eng_is_ff() ? 0 : q == 8 ? 2 : q == 9 ? 1 : 0; }
+constexpr int sweep_eb5_dpar(int q) { return q == 9 ? 3 : 1; }
 
 template <int Q>
 int bk5_sweep_q(int F, const double* D, long long E, const void* u, const void* G, const void* mass,
@@ -155,7 +180,7 @@ int bk5_sweep_q(int F, const double* D, long long E, const void* u, const void* 
     const bool eo = (F == 6) && make_eo<typename Eng::C, Q>(D, false, prm.eo, &Eng::coef) &&
                     make_eo<typename Eng::C, Q>(D, true, prm.eot, &Eng::coef);
     if (eo) {
-        constexpr int DP = sweep_dpar5(Q) ? 2 : 0;
+        constexpr int DP = sweep_dpar5(Q);
         constexpr int EB = fit_eb5<Q, 6, DP ? sweep_eb5_dpar(Q) : sweep_eb5(Q), DP>();
         if (gform == BK_G_FF) {
             // G split ahead of time: the float-float engine's even-odd path
@@ -251,11 +276,12 @@ int bk3_launch(const P13<typename Eng::C, Q>& prm, long long E, const void* G, c
     return cudaGetLastError() == cudaSuccess ? BK_OK : BK_ERR_CUDA;
 }
 
-// direction-parallel gradient stages for the float-float engine at q = 6..9,
-// measured 8-94 % faster on GB300 (q = 8: 13.1 against 10.3 GDoF/s), with
-// their own elements per block
-constexpr bool sweep_dpar3(int q) { return eng_is_ff() && q >= 6 && q <= 9; }
-constexpr int sweep_eb3_dpar(int q) { return q == 8 ? 2 : 3; }
+// direction-parallel gradient stages for the float-float engine from q = 7,
+// with their own elements per block (us against one thread per line: q = 8
+// 629 / 673, q = 10 763 / 1424, where a block is one element; q = 7 is level,
+// 689 / 683, and keeps the shorter latency; q = 6 loses, 614 / 592)
+constexpr bool sweep_dpar3(int q) { return eng_is_ff() && q >= 7; }
+constexpr int sweep_eb3_dpar(int q) { return q == 8 ? 2 : q == 9 ? 3 : 1; }
 
 template <int Q, int EB>
 int bk3_q(const double* B, const double* D, long long E, const void* G, const void* k, const void* u, void* v,
@@ -301,15 +327,15 @@ int bk3adj_launch(const P13<typename Eng::C, Q>& prm, long long E, const void* G
     return cudaGetLastError() == cudaSuccess ? BK_OK : BK_ERR_CUDA;
 }
 
-// the direction-parallel gradient sweeps for the float-float engine
-constexpr bool adj_dpar(int q) { return eng_is_ff() && q >= 6 && q <= 9; }
-constexpr int adj_eb_dpar(int q) { return q <= 6 ? 2 : 1; }
+// the direction-parallel gradient sweeps for the float-float engine (q = 6
+// 772 us against 930 with one thread per line, q = 10 1050 against 2845)
+constexpr bool adj_dpar(int q) { return eng_is_ff() && q >= 6; }
 
 template <int Q>
 int bk3adj_q(const double* B, const double* D, long long E, const void* G, const void* k, const void* u,
              const void* res, void* dk, void* dG, int gform, cudaStream_t s)
 {
-    constexpr int EB = default_eb(Q) / 2 > 0 ? default_eb(Q) / 2 : 1;
+    constexpr int EB = adj_eb(Q);
     P13<typename Eng::C, Q> prm;
     for (int i = 0; i < (Q - 1) * Q; ++i) prm.B[i] = Eng::coef(B[i]);
     for (int i = 0; i < Q * Q; ++i) prm.D[i] = Eng::coef(D[i]);
@@ -318,10 +344,10 @@ int bk3adj_q(const double* B, const double* D, long long E, const void* G, const
         if (gform == BK_G_FF) {
             // G split ahead of time: the float-float engine's even-odd path
             if constexpr (eng_is_ff())
-                return bk3adj_launch<Q, DP ? adj_eb_dpar(Q) : EB, true, DP, ff2>(prm, E, G, k, u, res, dk, dG, s);
+                return bk3adj_launch<Q, EB, true, DP, ff2>(prm, E, G, k, u, res, dk, dG, s);
             return BK_ERR_PREC;
         }
-        return bk3adj_launch<Q, DP ? adj_eb_dpar(Q) : EB, true, DP>(prm, E, G, k, u, res, dk, dG, s);
+        return bk3adj_launch<Q, EB, true, DP>(prm, E, G, k, u, res, dk, dG, s);
     }
     if (gform != BK_G_STORAGE) return BK_ERR_PREC;
     return bk3adj_launch<Q, EB, false, 0>(prm, E, G, k, u, res, dk, dG, s);
@@ -373,26 +399,19 @@ int BK_CAT3(bk5_col, BK_SFX, BK_LAYOUT_TU)(int p, int F, int eb, const double* D
 #endif
 
 #if BK_OP_TU == 1
-// Elements per BK1 block: the default (about 128 lines) except the
-// FP32-storage forms at q = 5 (BK1 p=3), whose EB = 5 (125 lines in 128
-// threads) measured fastest of EB = 1..10 on GB300: FP32 88.8 against 85.0
-// GDoF/s at E = 4096, 181.0 against 171.8 at E = 131072; the float-float
-// engine keeps EB = 6 (35.8 against 35.1, 52.1 against 50.4).
-constexpr int bk1_eb(int q) { return (q == 5 && !eng_is_ff() && !eng_is_dfma()) ? 5 : default_eb(q); }
-
 int BK_CAT(launch_bk1, BK_SFX)(int p, long long E, const double* B, const void* jxw, const void* u, void* v,
                                 int eb, int jxw_t, cudaStream_t s)
 {
     (void)eb;
     switch (p + 2) {
-        case 3: return bk1_q<3, default_eb(3)>(B, E, jxw, u, v, jxw_t, s);
-        case 4: return bk1_q<4, default_eb(4)>(B, E, jxw, u, v, jxw_t, s);
-        case 5: return bk1_q<5, bk1_eb(5)>(B, E, jxw, u, v, jxw_t, s);
-        case 6: return bk1_q<6, default_eb(6)>(B, E, jxw, u, v, jxw_t, s);
-        case 7: return bk1_q<7, default_eb(7)>(B, E, jxw, u, v, jxw_t, s);
-        case 8: return bk1_q<8, default_eb(8)>(B, E, jxw, u, v, jxw_t, s);
-        case 9: return bk1_q<9, default_eb(9)>(B, E, jxw, u, v, jxw_t, s);
-        case 10: return bk1_q<10, default_eb(10)>(B, E, jxw, u, v, jxw_t, s);
+        case 3: return bk1_q<3, sweep_eb1(3)>(B, E, jxw, u, v, jxw_t, s);
+        case 4: return bk1_q<4, sweep_eb1(4)>(B, E, jxw, u, v, jxw_t, s);
+        case 5: return bk1_q<5, sweep_eb1(5)>(B, E, jxw, u, v, jxw_t, s);
+        case 6: return bk1_q<6, sweep_eb1(6)>(B, E, jxw, u, v, jxw_t, s);
+        case 7: return bk1_q<7, sweep_eb1(7)>(B, E, jxw, u, v, jxw_t, s);
+        case 8: return bk1_q<8, sweep_eb1(8)>(B, E, jxw, u, v, jxw_t, s);
+        case 9: return bk1_q<9, sweep_eb1(9)>(B, E, jxw, u, v, jxw_t, s);
+        case 10: return bk1_q<10, sweep_eb1(10)>(B, E, jxw, u, v, jxw_t, s);
         default: return BK_ERR_ORDER;
     }
 }
