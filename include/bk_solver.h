@@ -24,7 +24,8 @@ typedef struct bk_order_range {
     int64_t E;           /* elements of this order */
     int elems_per_tile;  /* elements per tile of the persistent launch, with
                             elems_per_tile * q^2 <= 1024 (the column body:
-                            <= 256, one thread per column); 0: about 128 / q^2 */
+                            <= 256, one thread per column); 0: the library's
+                            own (28, 16, 5, 3, 2, 2, 1 for p = 2..8) */
 } bk_order_range;
 
 typedef struct bk_hplan* bk_hplan_t;
@@ -53,7 +54,7 @@ int bk_hplan_set_kernel(bk_hplan_t plan, int kernel);
 
 /* The shape of the even-odd sweep body's persistent launch.  threads: per
  * block, a multiple of 32 in 64..256, or 0 (the default) for the largest
- * tile's lines (elements x q^2, at most 256); tiles with more lines than
+ * tile's lines (elements x q^2, at most 128); tiles with more lines than
  * threads loop over their lines, so tile sizes per order and the block are
  * chosen apart.  The FP64 launch runs three thread groups of that size (one
  * per direction).  gstage (FP32 storage): 1 stages each tile's G into shared

@@ -34,12 +34,25 @@ namespace bkg {
 namespace {
 
 constexpr int kNT = 256;   // threads per block of the persistent kernel (per thread group), at most
+constexpr int kDefThreads = 128;  // threads of the sweep launch (per group) unless the plan sets them
 constexpr int kMaxTileLines = 1024;   // lines (elements x q^2) of a tile, at most
+// Elements per tile of the orders p = 2..8 unless the plan sets them: the
+// autotuner's picks at 5 M to 43 M points, mixed and float-float, but 28
+// instead of 42 at p = 2 (the column body, one thread per column, takes 256),
+// in blocks of kDefThreads.  Against ceil(128 / q^2) elements in blocks of the
+// largest tile's lines, p = 2..8, 43.5 M points: mixed 414 -> 340 us,
+// float-float 2494 -> 1530.
+constexpr int kDefTile[7] = {28, 16, 5, 3, 2, 2, 1};
 constexpr int kRedBlocks = 1216;   // 8 blocks of 256 threads per SM
 constexpr int kMaxDotParts = 4864;  // blocks of the persistent launch at most (32 per SM)
 constexpr int kRedThreads = 256;
+// The two vector kernels of the inner CG: two blocks of 512 threads per SM.
+// Fewer, larger blocks than the reductions' because each block first sums the
+// previous kernel's partials in FP64 (1/64 of the FP32 rate).
+constexpr int kCgBlocks = 304;
+constexpr int kCgThreads = 512;
 
-enum Scalar { S_RR = 0, S_RR0, S_PAP, S_IT, S_TOL2, S_MAXIT, S_NORM, S_INV, S_RN2, S_FN2, S_NSCAL };
+enum Scalar { S_RR = 0, S_RR0, S_RRN, S_ALPHA, S_IT, S_TOL2, S_MAXIT, S_NORM, S_INV, S_RN2, S_FN2, S_NSCAL };
 
 template <class Eng, int NBUF>
 struct MultiLaunch {
@@ -99,7 +112,8 @@ struct MultiLaunch {
 };
 
 // The even-odd sweep launch: blockDim = the largest tile's lines (eb q^2),
-// rounded up to whole warps, or the plan's block size when that is smaller
+// rounded up to whole warps, or the plan's block size (kDefThreads by default)
+// when that is smaller
 // (the sweeps of a tile with more lines than threads loop over them); three
 // times that with direction-parallel groups (DPAR); MAXT threads at most,
 // MINB blocks per SM asked of the register allocator.  GST: FP32 G staged.
@@ -112,7 +126,8 @@ struct MultiEOLaunch {
             const int l = (seg[s].eb * seg[s].q * seg[s].q + 31) / 32 * 32;
             nt = l > nt ? l : nt;
         }
-        if (block > 0 && nt > block) nt = block;
+        const int most = block > 0 ? block : kDefThreads;
+        if (nt > most) nt = most;
         if (DPAR) nt *= 3;
         return nt > MAXT ? MAXT : nt;
     }
@@ -279,12 +294,13 @@ __global__ void cg_start_kernel(long long n, const double* __restrict__ r64, con
 // loops run over float4 groups (one 16-byte load per vector and thread and
 // iteration, enough bytes in flight for HBM) and a scalar tail of n % 4.
 
+template <int NT = kRedThreads>
 __device__ __forceinline__ double block_reduce(double s)
 {
-    __shared__ double sh[kRedThreads];
+    __shared__ double sh[NT];
     sh[threadIdx.x] = s;
     __syncthreads();
-    for (int w = kRedThreads / 2; w > 0; w >>= 1) {
+    for (int w = NT / 2; w > 0; w >>= 1) {
         if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
         __syncthreads();
     }
@@ -313,14 +329,15 @@ __global__ void __launch_bounds__(kRedThreads) red_dot_kernel(long long n, const
     if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
 
+template <int NT = kRedThreads>
 __device__ __forceinline__ double block_sum(const double* __restrict__ part, int nb)
 {
-    __shared__ double sh[kRedThreads];
+    __shared__ double sh[NT];
     double s = 0.0;
-    for (int i = threadIdx.x; i < nb; i += kRedThreads) s += part[i];
+    for (int i = threadIdx.x; i < nb; i += NT) s += part[i];
     sh[threadIdx.x] = s;
     __syncthreads();
-    for (int w = kRedThreads / 2; w > 0; w >>= 1) {
+    for (int w = NT / 2; w > 0; w >>= 1) {
         if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
         __syncthreads();
     }
@@ -335,97 +352,132 @@ __global__ void __launch_bounds__(kRedThreads) cg_init_scalars_kernel(const doub
     if (threadIdx.x == 0) {
         sc[S_RR] = rr;
         sc[S_RR0] = rr;
+        sc[S_RRN] = rr;
         sc[S_IT] = 0.0;
     }
 }
 
-__global__ void __launch_bounds__(kRedThreads) cg_pap_kernel(const double* __restrict__ part, int nb,
-                                                             double* __restrict__ sc)
+// An iteration of the inner CG is three kernels: the apply (with the partial
+// sums of p.Ap), cg_update_kernel and cg_dir_kernel.  Each block of the last
+// two first sums the previous kernel's partials itself (about 10 KB from L2,
+// in one fixed order, so every block has the same bits), instead of a
+// one-block kernel between them.  d is updated with the new direction, where
+// p is read anyway: 10 instead of 11 vector reads and writes an iteration.
+//
+// Scalars: every block reads the ones its kernel needs, and block 0 writes
+// only such as no block of the same kernel reads.
+
+// r -= alpha Ap at four points and their terms of r.z (z = w .* r) into t,
+// each product exact and the sum compensated (acc_madd_f)
+__device__ __forceinline__ float4 cg_update4(float alpha, const float4& aa, float4 rr, const float4& w, ffacc& t)
 {
-    const double pap = block_sum(part, nb);
-    if (threadIdx.x == 0) sc[S_PAP] = pap;
+    rr.x = fmaf(-alpha, aa.x, rr.x);
+    rr.y = fmaf(-alpha, aa.y, rr.y);
+    rr.z = fmaf(-alpha, aa.z, rr.z);
+    rr.w = fmaf(-alpha, aa.w, rr.w);
+    acc_madd_f(t, rr.x, __fmul_rn(w.x, rr.x));
+    acc_madd_f(t, rr.y, __fmul_rn(w.y, rr.y));
+    acc_madd_f(t, rr.z, __fmul_rn(w.z, rr.z));
+    acc_madd_f(t, rr.w, __fmul_rn(w.w, rr.w));
+    return rr;
 }
 
-// d += alpha p, r -= alpha Ap and the partial sums of r.z = r.(invd .* r)
-// (the preconditioned CG's r.z; r.r without the preconditioner, invd = 1)
-__global__ void __launch_bounds__(kRedThreads) cg_update_kernel(long long n, const double* __restrict__ sc,
-                                                                const float* __restrict__ p,
-                                                                const float* __restrict__ Ap, float* __restrict__ d,
-                                                                float* __restrict__ r, const float* __restrict__ invd,
-                                                                double* __restrict__ part)
+// alpha = r.z / p.Ap, r -= alpha Ap and the partial sums of the new r.z =
+// r.(invd .* r) (r.r without the preconditioner, invd = 1).  part: the nb
+// partials of p.Ap; rpart: out.  The terms of eight points are summed in
+// float-float (2^-48 of their sum, which is of one sign) before they join the
+// thread's FP64 sum: with two conversions and an FP64 fma per point the FP64
+// pipe bounded the kernel (32 us of its 38 at 5.4 M points).
+__global__ void __launch_bounds__(kCgThreads) cg_update_kernel(long long n, double* __restrict__ sc,
+                                                               const double* __restrict__ part, int nb,
+                                                               const float* __restrict__ Ap, float* __restrict__ r,
+                                                               const float* __restrict__ invd,
+                                                               double* __restrict__ rpart)
 {
-    const double pap = sc[S_PAP];
-    const float alpha = float(pap != 0.0 ? sc[S_RR] / pap : 0.0);
-    const long long n4 = n / 4;
-    const long long stride = (long long)gridDim.x * kRedThreads;
-    double s = 0.0;
-    for (long long i = blockIdx.x * (long long)kRedThreads + threadIdx.x; i < n4; i += stride) {
-        const float4 pp = reinterpret_cast<const float4*>(p)[i];
-        const float4 aa = reinterpret_cast<const float4*>(Ap)[i];
-        float4 dd = reinterpret_cast<float4*>(d)[i];
-        float4 rr = reinterpret_cast<float4*>(r)[i];
-        dd.x = fmaf(alpha, pp.x, dd.x);
-        dd.y = fmaf(alpha, pp.y, dd.y);
-        dd.z = fmaf(alpha, pp.z, dd.z);
-        dd.w = fmaf(alpha, pp.w, dd.w);
-        rr.x = fmaf(-alpha, aa.x, rr.x);
-        rr.y = fmaf(-alpha, aa.y, rr.y);
-        rr.z = fmaf(-alpha, aa.z, rr.z);
-        rr.w = fmaf(-alpha, aa.w, rr.w);
-        reinterpret_cast<float4*>(d)[i] = dd;
-        reinterpret_cast<float4*>(r)[i] = rr;
-        const float4 w = reinterpret_cast<const float4*>(invd)[i];
-        s = fma(double(rr.x), double(w.x * rr.x), s);
-        s = fma(double(rr.y), double(w.y * rr.y), s);
-        s = fma(double(rr.z), double(w.z * rr.z), s);
-        s = fma(double(rr.w), double(w.w * rr.w), s);
+    const double pap = block_sum<kCgThreads>(part, nb);
+    const double rz = sc[S_RRN];
+    const float alpha = float(pap != 0.0 ? rz / pap : 0.0);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        sc[S_RR] = rz;
+        sc[S_ALPHA] = double(alpha);
     }
-    for (long long i = 4 * n4 + blockIdx.x * (long long)kRedThreads + threadIdx.x; i < n; i += stride) {
-        d[i] = fmaf(alpha, p[i], d[i]);
+    const long long n4 = n / 4;
+    const long long stride = (long long)gridDim.x * kCgThreads;
+    const float4* a4 = reinterpret_cast<const float4*>(Ap);
+    const float4* w4 = reinterpret_cast<const float4*>(invd);
+    float4* r4 = reinterpret_cast<float4*>(r);
+    double s = 0.0;
+    for (long long i = blockIdx.x * (long long)kCgThreads + threadIdx.x; i < n4; i += 2 * stride) {
+        const long long j = i + stride;
+        const bool two = j < n4;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 a0 = a4[i], r0 = r4[i], w0 = w4[i];
+        const float4 a1 = two ? a4[j] : zero, r1 = two ? r4[j] : zero, w1 = two ? w4[j] : zero;
+        ffacc t = acc_zero();
+        r4[i] = cg_update4(alpha, a0, r0, w0, t);
+        const float4 q = cg_update4(alpha, a1, r1, w1, t);
+        if (two) r4[j] = q;
+        s += double(t.s) + double(t.c);
+    }
+    for (long long i = 4 * n4 + blockIdx.x * (long long)kCgThreads + threadIdx.x; i < n; i += stride) {
         const float ri = fmaf(-alpha, Ap[i], r[i]);
         r[i] = ri;
         s = fma(double(ri), double(invd[i] * ri), s);
     }
-    const double t = block_reduce(s);
-    if (threadIdx.x == 0) part[blockIdx.x] = t;
+    const double t = block_reduce<kCgThreads>(s);
+    if (threadIdx.x == 0) rpart[blockIdx.x] = t;
 }
 
-// rr_new, beta, iteration count and the loop condition
-__global__ void __launch_bounds__(kRedThreads) cg_step_kernel(const double* __restrict__ part, int nb,
-                                                              double* __restrict__ sc, double* __restrict__ beta_out,
-                                                              cudaGraphConditionalHandle handle)
+// beta = new r.z / old r.z, d += alpha p, p = z + beta p with z = invd .* r;
+// block 0 counts the iteration and sets the loop condition.
+__global__ void __launch_bounds__(kCgThreads) cg_dir_kernel(long long n, double* __restrict__ sc,
+                                                             const double* __restrict__ rpart, int nb,
+                                                             const float* __restrict__ r,
+                                                             const float* __restrict__ invd, float* __restrict__ p,
+                                                             float* __restrict__ d, cudaGraphConditionalHandle handle)
 {
-    const double rr = block_sum(part, nb);
-    if (threadIdx.x == 0) {
-        const double old = sc[S_RR];
-        beta_out[0] = old != 0.0 ? rr / old : 0.0;
-        sc[S_RR] = rr;
+    const double rr = block_sum<kCgThreads>(rpart, nb);
+    const double old = sc[S_RR];
+    const float beta = float(old != 0.0 ? rr / old : 0.0);
+    const float alpha = float(sc[S_ALPHA]);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        sc[S_RRN] = rr;
         const double it = sc[S_IT] + 1.0;
         sc[S_IT] = it;
         const bool go = (rr > sc[S_TOL2] * sc[S_RR0]) && (it < sc[S_MAXIT]);
         cudaGraphSetConditional(handle, go ? 1u : 0u);
     }
-}
-
-// p = z + beta p, z = invd .* r
-__global__ void cg_dir_kernel(long long n, const double* __restrict__ beta_in, const float* __restrict__ r,
-                              const float* __restrict__ invd, float* __restrict__ p)
-{
-    const float beta = float(beta_in[0]);
     const long long n4 = n / 4;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += stride) {
-        const float4 rr = reinterpret_cast<const float4*>(r)[i];
-        const float4 w = reinterpret_cast<const float4*>(invd)[i];
-        float4 pp = reinterpret_cast<float4*>(p)[i];
-        pp.x = fmaf(beta, pp.x, w.x * rr.x);
-        pp.y = fmaf(beta, pp.y, w.y * rr.y);
-        pp.z = fmaf(beta, pp.z, w.z * rr.z);
-        pp.w = fmaf(beta, pp.w, w.w * rr.w);
-        reinterpret_cast<float4*>(p)[i] = pp;
+    const long long stride = (long long)gridDim.x * kCgThreads;
+    const float4* r4 = reinterpret_cast<const float4*>(r);
+    const float4* w4 = reinterpret_cast<const float4*>(invd);
+    float4* p4 = reinterpret_cast<float4*>(p);
+    float4* d4 = reinterpret_cast<float4*>(d);
+    auto step = [&](long long i, const float4& rv, const float4& w, float4 pp, float4 dd) {
+        dd.x = fmaf(alpha, pp.x, dd.x);
+        dd.y = fmaf(alpha, pp.y, dd.y);
+        dd.z = fmaf(alpha, pp.z, dd.z);
+        dd.w = fmaf(alpha, pp.w, dd.w);
+        d4[i] = dd;
+        pp.x = fmaf(beta, pp.x, w.x * rv.x);
+        pp.y = fmaf(beta, pp.y, w.y * rv.y);
+        pp.z = fmaf(beta, pp.z, w.z * rv.z);
+        pp.w = fmaf(beta, pp.w, w.w * rv.w);
+        p4[i] = pp;
+    };
+    long long i = blockIdx.x * (long long)kCgThreads + threadIdx.x;
+    for (; i + stride < n4; i += 2 * stride) {
+        const long long j = i + stride;
+        const float4 r0 = r4[i], w0 = w4[i], p0 = p4[i], d0 = d4[i];
+        const float4 r1 = r4[j], w1 = w4[j], p1 = p4[j], d1 = d4[j];
+        step(i, r0, w0, p0, d0);
+        step(j, r1, w1, p1, d1);
     }
-    for (long long i = 4 * n4 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride)
-        p[i] = fmaf(beta, p[i], invd[i] * r[i]);
+    if (i < n4) step(i, r4[i], w4[i], p4[i], d4[i]);
+    for (long long k = 4 * n4 + blockIdx.x * (long long)kCgThreads + threadIdx.x; k < n; k += stride) {
+        d[k] = fmaf(alpha, p[k], d[k]);
+        p[k] = fmaf(beta, p[k], invd[k] * r[k]);
+    }
 }
 // x += |r| d (FP64), the norm from the scalars
 __global__ void cg_correct_kernel(long long n, const double* __restrict__ sc, const float* __restrict__ d,
@@ -533,8 +585,8 @@ struct bk_hplan {
     float* d32;
     float* invd;        // the inner CG's Jacobi preconditioner (ones without it)
     double* part;
+    double* rpart;      // partials of r.z
     double* sc;
-    double* beta;
     cudaGraphExec_t inner_exec;
     cudaGraph_t inner_graph;
     const void* g_key[3];   // operator pointers the graph was built for
@@ -640,8 +692,8 @@ void free_graph(bk_hplan* h)
     h->inner_graph = nullptr;
 }
 
-// The inner CG as a graph: start, r.r, then WHILE(cond) { A p, p.Ap, update,
-// step (sets cond), new direction }.
+// The inner CG as a graph: start, r.r, then WHILE(cond) { A p with p.Ap,
+// update, new direction (sets cond) }.
 // invd = 1 / diag(A) from the FP32 operator (precond), or ones.
 int fill_precond(bk_hplan* h, const void* G32, const void* mass32, double lambda, int precond, cudaStream_t s)
 {
@@ -733,22 +785,19 @@ int build_inner_graph(bk_hplan* h, const void* G32, const void* mass32, double l
                 cudaSuccess) {
                 rc = BK_ERR_CUDA;
             } else {
-                int arc;
+                int arc, nparts = kRedBlocks;
                 if (h->kernel == BK_KERNEL_SWEEP) {
                     // p . Ap summed by the apply itself (one partial per block)
-                    int nparts = 0;
                     arc = run_f32<EngMixed, true>(h->e_f32, h->tiles, h->ntiles, h->p32, G32, mass32, lambda, h->Ap32,
                                                   s, h->part, &nparts);
-                    cg_pap_kernel<<<1, kRedThreads, 0, s>>>(h->part, nparts, h->sc);
                 } else {
                     arc = apply_plan(h, 3, G32, mass32, lambda, h->p32, h->Ap32, s);
                     red_dot_kernel<<<kRedBlocks, kRedThreads, 0, s>>>(n, h->p32, h->Ap32, h->part);
-                    cg_pap_kernel<<<1, kRedThreads, 0, s>>>(h->part, kRedBlocks, h->sc);
                 }
-                cg_update_kernel<<<kRedBlocks, kRedThreads, 0, s>>>(n, h->sc, h->p32, h->Ap32, h->d32, h->r32,
-                                                                    h->invd, h->part);
-                cg_step_kernel<<<1, kRedThreads, 0, s>>>(h->part, kRedBlocks, h->sc, h->beta, handle);
-                cg_dir_kernel<<<gn, 256, 0, s>>>(n, h->beta, h->r32, h->invd, h->p32);
+                cg_update_kernel<<<kCgBlocks, kCgThreads, 0, s>>>(n, h->sc, h->part, nparts, h->Ap32, h->r32,
+                                                                    h->invd, h->rpart);
+                cg_dir_kernel<<<kCgBlocks, kCgThreads, 0, s>>>(n, h->sc, h->rpart, kCgBlocks, h->r32, h->invd, h->p32,
+                                                         h->d32, handle);
                 cudaGraph_t body_out = nullptr;
                 if (cudaStreamEndCapture(s, &body_out) != cudaSuccess || arc != BK_OK) rc = BK_ERR_CUDA;
             }
@@ -792,7 +841,7 @@ int bk_hplan_create(bk_hplan_t* out, int norders, const bk_order_range* orders, 
         }
         const int q = p + 1;
         int eb = orders[s].elems_per_tile;
-        if (eb <= 0) eb = (q * q >= 100) ? 1 : ((q * q >= 64) ? 2 : (128 + q * q - 1) / (q * q));
+        if (eb <= 0) eb = kDefTile[p - 2];
         if (eb * q * q > kMaxTileLines || orders[s].E < 0 || !D[s]) {
             delete h;
             return orders[s].E < 0 ? BK_ERR_SIZE : BK_ERR_ARG;
@@ -831,7 +880,7 @@ int bk_hplan_create(bk_hplan_t* out, int norders, const bk_order_range* orders, 
     rc |= ck(cudaMalloc(&h->invd, 4 * (nb + 4)));
     rc |= ck(cudaMalloc(&h->part, 8 * (kRedBlocks > kMaxDotParts ? kRedBlocks : kMaxDotParts)));
     rc |= ck(cudaMalloc(&h->sc, 8 * S_NSCAL));
-    rc |= ck(cudaMalloc(&h->beta, 8 * 2));
+    rc |= ck(cudaMalloc(&h->rpart, 8 * kCgBlocks));
     if (rc == BK_OK && h->ntiles > 0)
         rc = ck(cudaMemcpyAsync(h->tiles, h->htiles.data(), sizeof(MultiTile) * h->ntiles, cudaMemcpyHostToDevice, s));
     if (rc == BK_OK) rc = ck(cudaStreamSynchronize(s));
@@ -857,7 +906,7 @@ int bk_hplan_destroy(bk_hplan_t h)
     cudaFree(h->invd);
     cudaFree(h->part);
     cudaFree(h->sc);
-    cudaFree(h->beta);
+    cudaFree(h->rpart);
     delete h;
     return BK_OK;
 }

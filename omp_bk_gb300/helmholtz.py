@@ -62,10 +62,9 @@ def _declare():
 
 
 def default_tiles(p: int) -> int:
-    """Elements per tile when no tuning is given (the library's own default):
-    about 128 lines of (p+1) points, at least one element."""
-    q2 = (p + 1) ** 2
-    return 1 if q2 >= 100 else (2 if q2 >= 64 else (128 + q2 - 1) // q2)
+    """Elements per tile when no tuning is given (the library's own default),
+    p = 2..8."""
+    return (28, 16, 5, 3, 2, 2, 1)[p - 2]
 
 
 class HelmholtzPlan:
@@ -104,7 +103,7 @@ class HelmholtzPlan:
 
     def set_shape(self, block: int = 0, gstage: int = 0):
         """Threads per block of the sweep body's launch (0: the largest
-        tile's lines; tiles with more lines loop over them) and, for FP32
+        tile's lines, at most 128; tiles with more lines loop over them) and, for FP32
         storage, whether G is staged in shared memory (bk_hplan_set_shape)."""
         check(_declare().bk_hplan_set_shape(self.h, int(block), int(gstage)), "bk_hplan_set_shape")
 
