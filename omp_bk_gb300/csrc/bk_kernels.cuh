@@ -234,6 +234,33 @@ constexpr int stage_bytes(int n)
     return ((n * int(sizeof(S)) + 15) / 16) * 16 + 16;
 }
 
+// Q consecutive staged values (a k line of an element's data) into
+// registers.  Lines of threads with consecutive j are Q values apart, so for
+// even Q scalar loads meet in the same banks (8-way at 4-byte Q = 8); 128-bit
+// loads where every line starts on 16 bytes (the array does, and an element
+// is a whole number of such units), 64-bit ones where it starts on 8, take a
+// quarter or half of the wavefronts.  BK1 p=6 FP32 (with the swizzled box)
+// 166 -> 132 us at E = 120000, p=2 FP64 283 -> 263 at E = 500000.
+template <class S, int Q>
+__device__ __forceinline__ void stage_line(const S* src, S (&x)[Q])
+{
+    constexpr int B = Q * int(sizeof(S));   // bytes of a line
+    if constexpr (B % 8 == 0 && sizeof(S) < (B % 16 == 0 ? 16 : 8)) {
+        using T = typename std::conditional<B % 16 == 0, uint4, uint2>::type;
+        constexpr int N = int(sizeof(T) / sizeof(S));
+#pragma unroll
+        for (int c = 0; c < Q / N; ++c) {
+            alignas(16) S t[N];
+            *reinterpret_cast<T*>(t) = *reinterpret_cast<const T*>(src + c * N);
+#pragma unroll
+            for (int n = 0; n < N; ++n) x[c * N + n] = t[n];
+        }
+    } else {
+#pragma unroll
+        for (int n = 0; n < Q; ++n) x[n] = src[n];
+    }
+}
+
 // Issues the copy of src[0, n) (global) into the shared buffer `buf`
 // (16-byte aligned, stage_bytes(n) long).  Returns where src[0] lands.
 // `lim` is the end of the source array, whose start is 16-byte aligned: the
@@ -1236,7 +1263,7 @@ template <class Eng, int Q, int EB>
 struct BK1Cfg {
     using S = typename Eng::S;
     using V = typename Eng::V;
-    using WB = WBox3<Q, V>;
+    using WB = WBox3<Q, V, true>;   // swizzled rows at 4-byte Q = 8 (bk3_swz)
     static constexpr int P = Q - 1;
     static constexpr int Q3 = Q * Q * Q;
     static constexpr int P3 = P * P * P;
@@ -1323,13 +1350,13 @@ __global__ void __launch_bounds__(BK1Cfg<Eng, Q, EB>::NT)
 #pragma unroll
                     for (int o = 0; o < Q; ++o) y[o] = Eng::mul(y[o], Eng::load(jl[o * Q * Q]));
                 } else {
-                    const S* jl = js + e * Q3 + (i * Q + j) * Q;
+                    S jv[Q];
+                    stage_line<S, Q>(js + e * Q3 + (i * Q + j) * Q, jv);
 #pragma unroll
-                    for (int o = 0; o < Q; ++o) y[o] = Eng::mul(y[o], Eng::load(jl[o]));
+                    for (int o = 0; o < Q; ++o) y[o] = Eng::mul(y[o], Eng::load(jv[o]));
                 }
                 eor_line<Eng, Q, P, +1>(y, z, prm.bb);
-#pragma unroll
-                for (int o = 0; o < P; ++o) W0[la(o)] = z[o];
+                line_store<WB, P>(W0, la, z);
             });
             __syncthreads();
             if (bt + gridDim.x < nbatch) issue(bt + gridDim.x);   // the stage is free
