@@ -16,6 +16,7 @@ There is no CPU fallback: without the built library every call raises.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 from dataclasses import dataclass
 
@@ -87,11 +88,11 @@ def lib():
         "bk1_apply": [C.c_int, _i64, _dp, _vp, _vp, _vp, C.c_int, _vp],
         "bk3_apply": [C.c_int, _i64, _dp, _dp, _vp, _vp, _vp, C.c_int, _vp],
         "bk5_apply": [C.c_int, _i64, _dp, _vp, _vp, _vp, C.c_int, _vp],
-        "bk1_apply_opt": [C.c_int, _i64, _dp, _vp, _vp, _vp, C.POINTER(Options), _vp],
+        "bk1_apply_opt": [C.c_int, _i64, _vp, _vp, _vp, _vp, C.POINTER(Options), _vp],
         "bk3_apply_opt": [C.c_int, _i64, _dp, _dp, _vp, _vp, _vp, C.POINTER(Options), _vp],
         "bk5_apply_opt": [C.c_int, _i64, _dp, _vp, _vp, _vp, C.POINTER(Options), _vp],
-        "bk5_apply_ex": [C.c_int, _i64, _dp, _vp, _vp, _vp, C.c_double, _vp, C.POINTER(Options), _vp],
-        "bk3_apply_k": [C.c_int, _i64, _dp, _dp, _vp, _vp, _vp, _vp, C.POINTER(Options), _vp],
+        "bk5_apply_ex": [C.c_int, _i64, _vp, _vp, _vp, _vp, C.c_double, _vp, C.POINTER(Options), _vp],
+        "bk3_apply_k": [C.c_int, _i64, _vp, _vp, _vp, _vp, _vp, _vp, C.POINTER(Options), _vp],
         "bk_device_status": [C.POINTER(C.c_int), C.c_int, _vp],
         "bk_set_wait_limit": [C.c_longlong],
         "bk_test_wait_timeout": [_vp],
@@ -108,7 +109,7 @@ def lib():
         "bk_geom_trilinear": [C.c_int, C.c_longlong, C.c_int, C.c_int, _dp, _dp, C.c_ulonglong, C.c_double,
                               C.c_double, _vp, C.c_int, _vp, _vp, _vp],
         "bk_convert": [_vp, _vp, C.c_longlong, C.c_int, _vp],
-        "bk3_adjoint": [C.c_int, _i64, _dp, _dp, _vp, _vp, _vp, _vp, _vp, _vp, C.POINTER(Options), _vp],
+        "bk3_adjoint": [C.c_int, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, C.POINTER(Options), _vp],
         "bk_stream_kernel": [C.c_int, C.c_longlong, _vp, _vp, _vp, C.c_int, _vp],
         "bk_dot": [C.c_longlong, _vp, _vp, C.c_int, _vp, _vp, C.c_longlong, C.c_int, _vp],
         "bk_axpby": [C.c_longlong, C.c_double, _vp, C.c_double, _vp, C.c_int, _vp],
@@ -138,6 +139,14 @@ def check(rc: int, what: str) -> None:
 
 # ---- helpers -------------------------------------------------------------------
 
+def _mat(a) -> tuple:
+    """A 1-D matrix as float64 in row-major order and its address (the array
+    is kept alive by the returned tuple); no copy of one that is already so."""
+    if not (type(a) is np.ndarray and a.dtype.char == "d" and a.dtype.isnative and a.flags.c_contiguous):
+        a = np.ascontiguousarray(np.asarray(a, dtype=np.float64))
+    return a, a.ctypes.data
+
+
 def _host(a) -> tuple:
     """A C double* to a contiguous float64 copy of `a` (kept alive by the
     returned tuple)."""
@@ -157,10 +166,27 @@ def _order(p: int, what: str) -> None:
         raise BKError(BK_ERR_ORDER, f"{what}: p = {p}")
 
 
+_raw_stream = None
+
+
+def _current_stream() -> int:
+    """The handle of torch's current stream on the current device.  Through
+    torch's raw-stream call where it has one: the Stream object of the public
+    call costs 4 us, a third of a small apply's time on the host."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        raw, dev = (getattr(torch._C, n, None) for n in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
+        if raw is None or dev is None:
+            return torch.cuda.current_stream().cuda_stream
+        torch.cuda.init()
+        _raw_stream = lambda: raw(dev())
+    return _raw_stream()
+
+
 def _stream(stream):
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream
+        return _current_stream()
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
@@ -188,6 +214,14 @@ class ApplyOptions:
                        self.gform, self.jxw_layout)
 
 
+@functools.lru_cache(maxsize=512, typed=True)
+def _opt(prec=PREC_FP64, engine=ENGINE_AUTO, layout=LAYOUT_INTERLEAVED, nfactors=6, elems_per_block=0,
+         kernel=KERNEL_AUTO, gform=G_STORAGE, jxw_layout=JXW_PQR):
+    """A reference to the bk_options of these values (read by the library
+    only, so one structure per set of values serves every call)."""
+    return C.byref(Options(prec, engine, layout, nfactors, elems_per_block, kernel, gform, jxw_layout))
+
+
 # ---- operator apply (device tensors) -------------------------------------------
 
 def bk1_apply(p, E, B, qdata, u, v, prec=PREC_FP64, engine=ENGINE_AUTO, jxw_layout=JXW_PQR, stream=None):
@@ -195,9 +229,9 @@ def bk1_apply(p, E, B, qdata, u, v, prec=PREC_FP64, engine=ENGINE_AUTO, jxw_layo
     jxw_layout=JXW_RQP: qdata is JxW_t(e, r, q, p), as bk1_transpose_jxw
     (transpose_jxw, include/bk_harness.h:89-102) makes it."""
     _order(p, "bk1_apply")
-    Bh, Bp = _host(B)
-    o = ApplyOptions(prec=prec, engine=engine, jxw_layout=jxw_layout).c()
-    check(lib().bk1_apply_opt(p, E, Bp, _ptr(qdata), _ptr(u), _ptr(v), C.byref(o), _stream(stream)), "bk1_apply")
+    Bh, Bp = _mat(B)
+    o = _opt(prec=prec, engine=engine, jxw_layout=jxw_layout)
+    check(lib().bk1_apply_opt(p, E, Bp, _ptr(qdata), _ptr(u), _ptr(v), o, _stream(stream)), "bk1_apply")
 
 
 def bk3_apply(p, E, B, D, G, u, v, k=None, prec=PREC_FP64, engine=ENGINE_AUTO, gform=G_STORAGE, stream=None):
@@ -205,10 +239,10 @@ def bk3_apply(p, E, B, D, G, u, v, k=None, prec=PREC_FP64, engine=ENGINE_AUTO, g
     factor-major, k an optional coefficient at the quadrature points.
     gform=G_FF: G holds the float-float pairs made by g_to_ff."""
     _order(p, "bk3_apply")
-    Bh, Bp = _host(B)
-    Dh, Dp = _host(D)
-    o = ApplyOptions(prec=prec, engine=engine, gform=gform).c()
-    check(lib().bk3_apply_k(p, E, Bp, Dp, _ptr(G), _ptr(k), _ptr(u), _ptr(v), C.byref(o), _stream(stream)),
+    Bh, Bp = _mat(B)
+    Dh, Dp = _mat(D)
+    o = _opt(prec=prec, engine=engine, gform=gform)
+    check(lib().bk3_apply_k(p, E, Bp, Dp, _ptr(G), _ptr(k), _ptr(u), _ptr(v), o, _stream(stream)),
           "bk3_apply")
 
 
@@ -217,10 +251,10 @@ def bk5_apply(p, E, D, G, u, v, prec=PREC_FP64, engine=ENGINE_AUTO, layout=LAYOU
     """v = D^T G D u (+ lam * mass * u) per element (openmp/BK5.cpp:18-103).
     gform=G_FF: G holds the float-float pairs made by g_to_ff."""
     _order(p, "bk5_apply")
-    Dh, Dp = _host(D)
-    o = ApplyOptions(prec=prec, engine=engine, layout=layout, nfactors=nfactors, kernel=kernel,
-                     elems_per_block=elems_per_block, gform=gform).c()
-    check(lib().bk5_apply_ex(p, E, Dp, _ptr(G), _ptr(u), _ptr(mass), float(lam), _ptr(v), C.byref(o),
+    Dh, Dp = _mat(D)
+    o = _opt(prec=prec, engine=engine, layout=layout, nfactors=nfactors, kernel=kernel,
+             elems_per_block=elems_per_block, gform=gform)
+    check(lib().bk5_apply_ex(p, E, Dp, _ptr(G), _ptr(u), _ptr(mass), float(lam), _ptr(v), o,
                              _stream(stream)), "bk5_apply")
 
 
@@ -417,10 +451,10 @@ def bk3_adjoint(p, E, B, D, G, k, u, res, dk, dG, prec=PREC_FP64, engine=ENGINE_
     res = A(k) u - f; the forward kernel is bk3_apply(..., k=k).  gform=G_FF:
     G holds the float-float pairs made by g_to_ff."""
     _order(p, "bk3_adjoint")
-    Bh, Bp = _host(B)
-    Dh, Dp = _host(D)
-    o = ApplyOptions(prec=prec, engine=engine, gform=gform).c()
-    check(lib().bk3_adjoint(p, E, Bp, Dp, _ptr(G), _ptr(k), _ptr(u), _ptr(res), _ptr(dk), _ptr(dG), C.byref(o),
+    Bh, Bp = _mat(B)
+    Dh, Dp = _mat(D)
+    o = _opt(prec=prec, engine=engine, gform=gform)
+    check(lib().bk3_adjoint(p, E, Bp, Dp, _ptr(G), _ptr(k), _ptr(u), _ptr(res), _ptr(dk), _ptr(dG), o,
                             _stream(stream)), "bk3_adjoint")
 
 

@@ -185,3 +185,30 @@ def test_tuner_candidates():
                     if max(1, k * block // q2) * q2 <= tune.MAX_TILE_LINES]
             assert set(full) == set(c)
         assert tune.candidates(p) == sorted({tune.tiles_for(p, t) for t in tune.LINE_BUDGETS})
+
+
+@pytest.mark.parametrize("make", [lambda a: a, lambda a: a.tolist(), lambda a: a.astype(np.float32),
+                                  lambda a: a.reshape(4, 3).T, lambda a: np.repeat(a, 2)[::2],
+                                  lambda a: a.astype(">f8")])
+def test_matrix_forms(make):
+    """A 1-D matrix may come as any array-like: the library gets float64 in
+    row-major order, without a copy where the array already is that."""
+    import omp_bk_gb300 as bk
+    src = make(np.arange(12, dtype=np.float64) / 7)
+    arr, ptr = bk._mat(src)
+    want = np.asarray(src, dtype=np.float64).ravel()
+    got = np.array((C.c_double * 12).from_address(ptr))
+    assert np.array_equal(got, want) and arr.dtype == np.float64 and arr.dtype.isnative
+    if isinstance(src, np.ndarray) and src.dtype == np.float64 and src.flags.c_contiguous:
+        assert arr is src
+
+
+def test_option_values_are_kept_apart():
+    """One options structure per set of values; a float in an option's place
+    is refused as before, also after the equal int was used."""
+    import omp_bk_gb300 as bk
+    a = bk._opt(prec=bk.PREC_FP32, layout=2)
+    assert bk._opt(prec=bk.PREC_FP32, layout=2) is a and bk._opt(prec=bk.PREC_MIXED, layout=2) is not a
+    assert (a._obj.prec, a._obj.layout, a._obj.nfactors) == (bk.PREC_FP32, 2, 6)
+    with pytest.raises(TypeError):
+        bk._opt(prec=float(bk.PREC_FP32), layout=2)

@@ -504,3 +504,25 @@ def test_fp64_factor_ranges(bklib, bk, p):
         bklib.bk3_apply(p, E, B, D, gd, ud, v)
     torch.cuda.synchronize()
     assert oracle.rel_maxdiff(host(v), ref) < TOL64
+
+
+def test_apply_runs_on_the_current_stream(bklib):
+    """Without a stream argument an apply is ordered with torch's work on the
+    current stream (here a side stream behind a long chain of fills)."""
+    p, E = 3, 3000
+    B, _, _, _, _ = bklib.bk1_bk3_matrices(p)
+    rng = np.random.default_rng(3)
+    u, q = rng.uniform(-1, 1, E * 64), rng.uniform(0.1, 1, E * 125)
+    ref = oracle.bk1(p + 2, E, np.asarray(B), q, u)
+    gq, src = dev(q, "f64"), dev(u, "f64")
+    gu, v = torch.zeros_like(src), torch.zeros_like(src)
+    big = torch.empty(1 << 27, device="cuda")
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        for k in range(8):
+            big.fill_(k)
+        gu.copy_(src)
+        bklib.bk1_apply(p, E, B, gq, gu, v)
+    s.synchronize()
+    assert oracle.rel_maxdiff(host(v), ref) < TOL64
