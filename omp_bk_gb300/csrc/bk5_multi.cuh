@@ -413,9 +413,11 @@ __global__ void __launch_bounds__(NT, MINB)
         const S* mb = (mass != nullptr) ? stage_at<S>(ust + u_bytes, mass + sg.uoff + tl.e_first * q3) : nullptr;
         // after the pointwise stage the G stage is free for the next tile's G
         auto early = [&]() {
+            __syncthreads();
             if constexpr (!GD) {
                 if (tn < ntiles) issue_g(tn, NB == 2 ? (b ^ 1) : 0, NB == 2);
             }
+            return false;
         };
         switch (q) {
 #define BK_MULTI_EO_CASE(QQ)                                                                                    \

@@ -33,7 +33,7 @@ struct BK3AdjCfg {
     static constexpr int G_BYTES = stage_bytes<S>(EB * 6 * Q3);
     static constexpr int K_BYTES = stage_bytes<S>(EB * Q3);
     static constexpr int W_BYTES = ((NBOX * EB * WB::size * int(sizeof(V)) + 15) / 16) * 16;
-    static constexpr int SMEM = 2 * U_BYTES + G_BYTES + K_BYTES + W_BYTES + 16;
+    static constexpr int SMEM = 2 * U_BYTES + G_BYTES + K_BYTES + W_BYTES + kTailBytes;
 };
 
 // u (P^3, dense S) -> gradient components at the Q^3 points in (gr, gs, gt);
@@ -41,11 +41,13 @@ struct BK3AdjCfg {
 // DPAR.  EO: the even-odd contractions of prm.bi (interpolation,
 // centro-symmetric) and prm.dg (derivative, centro-antisymmetric).  DPAR:
 // the three derivative sweeps at once on three thread groups of `lines`
-// threads, reading the interpolant from tmp.
+// threads, reading the interpolant from tmp.  Ends with a block barrier unless
+// end_sync is false.
 template <class Eng, class WB, int Q, bool EO, int DPAR = 0>
 __device__ __forceinline__ void grad_at_points(const typename Eng::S* src, typename Eng::V* tmp, typename Eng::V* gr,
                                                typename Eng::V* gs, typename Eng::V* gt, int ne,
-                                               const P13<typename Eng::C, Q>& prm, int tid, int nt, int lines = 0)
+                                               const P13<typename Eng::C, Q>& prm, int tid, int nt, int lines = 0,
+                                               const bool end_sync = true)
 {
     constexpr int P = Q - 1;
     const Mat<typename Eng::C, Q, true> Bi{prm.B};   // interpolation: M(p, i) = B[i*Q + p]
@@ -87,10 +89,11 @@ __device__ __forceinline__ void grad_at_points(const typename Eng::S* src, typen
         __syncthreads();
         sweep<Eng, WB, 2, Q, Q, Q, Q>(gt, gt, ne, Dg, tid, nt);
     }
-    __syncthreads();
+    if (end_sync) __syncthreads();
 }
 
-template <class Eng, int Q, int EB, bool EO = false, int DPAR = 0, class GS = typename Eng::S>
+template <class Eng, int Q, int EB, bool EO = false, int DPAR = 0, class GS = typename Eng::S,
+          bool DYN = false>
 __global__ void __launch_bounds__(BK3AdjCfg<Eng, Q, EB, DPAR>::NT)
     bk3_adjoint_kernel(const __grid_constant__ P13<typename Eng::C, Q> prm, const long long E,
                        const typename Eng::S* __restrict__ u, const typename Eng::S* __restrict__ res,
@@ -117,16 +120,12 @@ __global__ void __launch_bounds__(BK3AdjCfg<Eng, Q, EB, DPAR>::NT)
     V* W4 = W3 + EB * WB::size;
     V* W5 = W4 + EB * WB::size;
     V* W6 = DPAR ? W5 + EB * WB::size : W0;   // the third component of g_res
-    uint64_t* bar = reinterpret_cast<uint64_t*>(kstage + Cfg::K_BYTES + Cfg::W_BYTES);
     const int tid = threadIdx.x;
     const int nt = Cfg::NT;
 
-    if (tid == 0) {
-        mbar_init(bar, 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
     const long long nbatch = (E + EB - 1) / EB;
+    Walk<DYN> walk(kstage + Cfg::K_BYTES + Cfg::W_BYTES, nbatch, tid);
+    uint64_t* bar = walk.bar;
     // The next batch's u and res are copied as soon as both gradients are
     // formed (thread 0 adds their bytes to the phase without arriving), its
     // G and k once the products have read the current ones (thread 0
@@ -137,7 +136,7 @@ __global__ void __launch_bounds__(BK3AdjCfg<Eng, Q, EB, DPAR>::NT)
     const S* ks = nullptr;
     auto issue_ur = [&](long long bt, bool arrive) {
         const long long e0 = bt * EB;
-        const int ne = int((E - e0) < EB ? (E - e0) : EB);
+        const int ne = batch_elems<EB, S>(E, e0);
         uint32_t tx = 0;
         if (tid == 0) fence_proxy_async();
         us = stage_issue<S>(ustage, u + e0 * P3, ne * P3, u + E * P3, bar, tx, tid, nt);
@@ -151,7 +150,7 @@ __global__ void __launch_bounds__(BK3AdjCfg<Eng, Q, EB, DPAR>::NT)
     };
     auto issue_gk = [&](long long bt) {
         const long long e0 = bt * EB;
-        const int ne = int((E - e0) < EB ? (E - e0) : EB);
+        const int ne = batch_elems<EB, S>(E, e0);
         uint32_t tx = 0;
         if (tid == 0) fence_proxy_async();
         gs = stage_issue<GS>(gstage, G + e0 * 6 * Q3, ne * 6 * Q3, G + E * 6 * Q3, bar, tx, tid, nt);
@@ -163,16 +162,16 @@ __global__ void __launch_bounds__(BK3AdjCfg<Eng, Q, EB, DPAR>::NT)
         issue_gk(blockIdx.x);
     }
     uint32_t phase = 0;
-    for (long long bt = blockIdx.x; bt < nbatch; bt += gridDim.x, phase ^= 1u) {
+    for (long long bt = blockIdx.x < nbatch ? blockIdx.x : -1; bt >= 0; bt = walk.next, phase ^= 1u) {
         const long long e0 = bt * EB;
-        const int ne = int((E - e0) < EB ? (E - e0) : EB);
-        const long long next = bt + gridDim.x;
-        if (batch_wait_failed(bar, phase, ctx, tid)) return;
+        const int ne = batch_elems<EB, S>(E, e0);
+        if (walk.start(phase, ctx, tid)) return;
         // g_u -> (W1, W2, W3) with W0 as scratch; g_res -> (W4, W5, W6), W6 = W0
         // (its last use) unless DPAR
         grad_at_points<Eng, WB, Q, EO, DPAR>(us, W0, W1, W2, W3, ne, prm, tid, nt, Cfg::LINES);
-        grad_at_points<Eng, WB, Q, EO, DPAR>(rs, W0, W4, W5, W6, ne, prm, tid, nt, Cfg::LINES);
-        if (next < nbatch) issue_ur(next, false);   // u and res stages are free
+        grad_at_points<Eng, WB, Q, EO, DPAR>(rs, W0, W4, W5, W6, ne, prm, tid, nt, Cfg::LINES, false);
+        if (walk.advance(bt, phase, ctx, tid)) return;   // (a block barrier)
+        if (walk.next >= 0) issue_ur(walk.next, false);   // u and res stages are free
         for (int w = tid; w < ne * Q3; w += nt) {
             const int e = w / Q3;
             const int x = w - e * Q3;
@@ -214,7 +213,7 @@ __global__ void __launch_bounds__(BK3AdjCfg<Eng, Q, EB, DPAR>::NT)
             go[5 * Q3] = Eng::store(prod(kt, ut));
         }
         __syncthreads();
-        if (next < nbatch) issue_gk(next);
+        if (walk.next >= 0) issue_gk(walk.next);
     }
 }
 

@@ -130,6 +130,40 @@ __device__ __forceinline__ void tma_store_wait_all()
 
 __device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// ---- cluster launch control: the next block of the grid ------------------------
+//
+// A resident block takes over the work of a block of its grid that has not been
+// launched yet: clc_request asks for one (asynchronously; one arrival and the
+// 16 bytes of the answer on `bar`), clc_next decodes the answer: the block's
+// index, or -1 when none is left (after which no further request is made).
+struct alignas(16) ClcAnswer {
+    uint32_t w[4];
+};
+__device__ __forceinline__ void clc_request(ClcAnswer* a, uint64_t* bar)
+{
+    fence_proxy_async();   // the last answer has been read
+    mbar_arrive_expect_tx(bar, 16);
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                     smem_u32(a)),
+                 "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ long long clc_next(const ClcAnswer* a)
+{
+    uint32_t ok, x;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
+        "ld.shared.b128 h, [%2];\n\t"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "mov.u32 %1, 0;\n\t"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
+        : "=r"(ok), "=r"(x)
+        : "r"(smem_u32(a))
+        : "memory");
+    return ok ? static_cast<long long>(x) : -1;
+}
+
 // One arrival on the barrier (no transaction bytes).
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar)
 {

@@ -774,6 +774,75 @@ __device__ __forceinline__ bool batch_wait_failed(uint64_t* bar, uint32_t phase,
     return false;
 }
 
+// Elements of the batch that starts at element e0 < E; a constant for EB = 1
+// (the loops over elements vanish).  For FP32 storage (S) the compiler is told
+// the range, so that a loop over lines that the block's threads cover in one
+// step is none (BK1 p=1 176 -> 158 us, BK3 p=4 228 -> 220); the float-float
+// kernels were slower with it (adjoint p=4 729 -> 754, BK5 p=8 890 -> 950).
+template <int EB, class S>
+__device__ __forceinline__ int batch_elems(long long E, long long e0)
+{
+    if (EB == 1) return 1;
+    const int ne = int((E - e0) < EB ? (E - e0) : EB);
+    if constexpr (sizeof(S) == 4) __builtin_assume(ne >= 1 && ne <= EB);
+    return ne;
+}
+
+// How a block goes from batch to batch.
+//   DYN: the grid has a block per batch; a resident block takes over the
+//     batches of blocks not launched yet (cluster launch control), asked for
+//     at the start of a batch and known by the time its stages are free.  The
+//     blocks of an SM need not be equally fast: with 5 or 6 warps a block the
+//     four schedulers get uneven shares, and a static deal waits for the
+//     slowest (BK3 p=6 float-float 652 -> 577 us, BK5 p=7 716 -> 676, BK1 p=4
+//     FP32 179 -> 154).
+//   otherwise: batches blockIdx.x, + gridDim.x, ... of the resident blocks, for
+//     launches of a few waves, where the answers' latency shows.
+// A template parameter and not a flag of the launch: with a flag the compiler
+// kept more registers over the batch (adjoint p=4 729 -> 766 us).
+// The tail of a block's shared memory: the data barrier, the walk's, and its
+// answer.
+constexpr int kTailBytes = 32;
+template <bool DYN>
+struct Walk {
+    uint64_t* bar;    // the batch's copies
+    uint64_t* cbar;   // DYN: the answers
+    ClcAnswer* ans;
+    long long nbatch;
+    long long next;   // the next batch, -1: none (after advance())
+    __device__ __forceinline__ Walk(unsigned char* tail, long long nbatch_, int tid) : nbatch(nbatch_), next(-1)
+    {
+        bar = reinterpret_cast<uint64_t*>(tail);
+        cbar = bar + 1;
+        ans = reinterpret_cast<ClcAnswer*>(tail + 16);
+        if (tid == 0) {
+            mbar_init(bar, 1);
+            if (DYN) mbar_init(cbar, 1);
+            fence_mbar_init();
+        }
+        __syncthreads();
+    }
+    // waits for the batch's copies; true on a timeout (batch_wait_failed)
+    __device__ __forceinline__ bool start(uint32_t phase, const DevCtx& ctx, int tid) const
+    {
+        if (batch_wait_failed(bar, phase, ctx, tid)) return true;
+        if (DYN && tid == 0) clc_request(ans, cbar);
+        return false;
+    }
+    // A block barrier after which `next` is known; true on a timeout.
+    __device__ __forceinline__ bool advance(long long bt, uint32_t phase, const DevCtx& ctx, int tid)
+    {
+        if constexpr (DYN) {
+            if (batch_wait_failed(cbar, phase, ctx, tid)) return true;
+            next = clc_next(ans);
+        } else {
+            __syncthreads();
+            next = bt + gridDim.x < nbatch ? bt + gridDim.x : -1;
+        }
+        return false;
+    }
+};
+
 // ---- kernel parameters ---------------------------------------------------------
 
 template <class C, int Q>
@@ -853,13 +922,14 @@ struct BK5Cfg {
     static constexpr int G_BYTES = stage_bytes<S>(EB * F * Q3);
     static constexpr int STAGE_BYTES = U_BYTES + G_BYTES;
     static constexpr int W_BYTES = ((NBOX * EB * WB::size * int(sizeof(V)) + 15) / 16) * 16;
-    static constexpr int SMEM = STAGE_BYTES + W_BYTES + 16;
+    static constexpr int SMEM = STAGE_BYTES + W_BYTES + kTailBytes;
     // resident blocks asked of the register allocator (DPAR): what shared
     // memory allows (1 KB per block is the system's), down to 56 registers a
-    // thread; the flux pass would take up to 107 and halve the blocks
+    // thread; the flux pass would take up to 107 and halve the blocks.  Left to
+    // the compiler for the one block per SM of q = 9 (943 -> 906 us)
     static constexpr int BY_SMEM = 233472 / (SMEM + 1024) < 1 ? 1 : 233472 / (SMEM + 1024);
     static constexpr int BY_REGS = 65536 / (NT * 56) < 1 ? 1 : 65536 / (NT * 56);
-    static constexpr int MINB = DPAR == 0 ? 1 : (BY_SMEM < BY_REGS ? BY_SMEM : BY_REGS);
+    static constexpr int MINB = DPAR == 0 ? 1 : LINES > 192 ? 0 : (BY_SMEM < BY_REGS ? BY_SMEM : BY_REGS);
 };
 
 // One batch of ne elements of order Q whose u (us, dense; shared or global
@@ -870,8 +940,10 @@ struct BK5Cfg {
 // or shared, may be NULL) with u at us.  DOT (FP32 storage): the thread's
 // running sum of u . v over its points in *dot, each product exact (FMA) and
 // the sum compensated (float-float: about 44 bits).  after_pw: called by every
-// thread after the pointwise stage, when the G stage is no longer read (nor
-// u, unless the mass term or dot reads it at the end).  Ends with a block
+// thread after the pointwise stage; a block barrier, behind which the G stage
+// is no longer read (nor u, unless the mass term or dot reads it at the end);
+// if it returns true (a wait gave up) the batch is left and true returned.
+// Ends with a block
 // barrier (after which the stages may be reused) unless end_sync is false.
 // GS: the type G is stored in (the storage type, or float-float pairs split
 // ahead of time).
@@ -889,13 +961,17 @@ struct BK5Cfg {
 // one code body per direction (strides known at compile time); DPAR = 2: one
 // body for all three, the direction's strides in registers (a third of the
 // instruction footprint of the stage).
-struct NoOp {
-    __device__ __forceinline__ void operator()() const {}
+struct SyncOnly {
+    __device__ __forceinline__ bool operator()() const
+    {
+        __syncthreads();
+        return false;
+    }
 };
 
-template <class Eng, int Q, int F, int LAYOUT, bool EO, int DPAR = 0, class AfterPw = NoOp, bool DOT = false,
+template <class Eng, int Q, int F, int LAYOUT, bool EO, int DPAR = 0, class AfterPw = SyncOnly, bool DOT = false,
           class GS = typename Eng::S>
-__device__ __forceinline__ void bk5_sweep_batch(const typename Eng::C* __restrict__ Dp,
+__device__ __forceinline__ bool bk5_sweep_batch(const typename Eng::C* __restrict__ Dp,
                                                 const EOMat<typename Eng::C, Q>& eo,
                                                 const EOMat<typename Eng::C, Q>& eot, const typename Eng::S* us,
                                                 const GS* gs, typename Eng::V* W0, typename Eng::V* W1,
@@ -1027,8 +1103,7 @@ __device__ __forceinline__ void bk5_sweep_batch(const typename Eng::C* __restric
             for (int n = 0; n < Q; ++n) flux(e, r, n);
         }
     }
-    __syncthreads();
-    after_pw();   // the G stage (and u, without a mass term) is free from here
+    if (after_pw()) return true;   // the G stage (and u, without a mass term) is free from here
     // 5. transposed derivatives, in place: along i on W0, along j on W1 and
     //    (even-odd) along k on QT
     if constexpr (DPAR == 2) {
@@ -1168,14 +1243,15 @@ __device__ __forceinline__ void bk5_sweep_batch(const typename Eng::C* __restric
     // end_sync (uniform): false when the caller's next step is a block
     // barrier anyway and nothing before it writes what the last pass read
     if (end_sync) __syncthreads();
+    return false;
 }
 
-// The block walks batches bt = blockIdx.x, + gridDim.x, ...  One stage buffer:
-// the next batch's u and G are copied into it as soon as the current batch
+// The block goes from batch to batch (Walk).  One stage buffer: the next batch's u and G are copied into it as soon as the current batch
 // stops reading them (after the pointwise stage; u after the last pass when a
 // mass term reads it there), so the copies overlap the transposed sweeps and
 // the last pass instead of stalling the block at the start of each batch.
-template <class Eng, int Q, int EB, int F, int LAYOUT, bool EO = false, int DPAR = 0, class GS = typename Eng::S>
+template <class Eng, int Q, int EB, int F, int LAYOUT, bool EO = false, int DPAR = 0, class GS = typename Eng::S,
+          bool DYN = false>
 __global__ void __launch_bounds__(BK5Cfg<Eng, Q, EB, F, LAYOUT, DPAR>::NT, BK5Cfg<Eng, Q, EB, F, LAYOUT, DPAR>::MINB)
     bk5_kernel(const __grid_constant__ P5<typename Eng::C, Q> prm, const long long E,
                const typename Eng::S* __restrict__ u, const GS* __restrict__ G,
@@ -1193,16 +1269,11 @@ __global__ void __launch_bounds__(BK5Cfg<Eng, Q, EB, F, LAYOUT, DPAR>::NT, BK5Cf
     V* W1 = W0 + EB * WB::size;
     V* W2 = W1 + EB * WB::size;
     V* W3 = DPAR ? W2 + EB * WB::size : nullptr;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + Cfg::STAGE_BYTES + Cfg::W_BYTES);
     const int tid = threadIdx.x;
     const int nt = Cfg::NT;
-
-    if (tid == 0) {
-        mbar_init(bar, 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
     const long long nbatch = (E + EB - 1) / EB;
+    Walk<DYN> walk(smem + Cfg::STAGE_BYTES + Cfg::W_BYTES, nbatch, tid);
+    uint64_t* bar = walk.bar;
     // where the staged batch's u and G landed
     const S* us = nullptr;
     const GS* gs = nullptr;
@@ -1211,7 +1282,7 @@ __global__ void __launch_bounds__(BK5Cfg<Eng, Q, EB, F, LAYOUT, DPAR>::NT, BK5Cf
     //    batch bt's phase completes when both have landed
     auto issue_g = [&](long long bt) {
         const long long e0 = bt * EB;
-        const int ne = int((E - e0) < EB ? (E - e0) : EB);
+        const int ne = batch_elems<EB, S>(E, e0);
         uint32_t tx = 0;
         if (tid == 0) fence_proxy_async();
         gs = stage_issue<GS>(smem + Cfg::U_BYTES, G + e0 * F * Q3, ne * F * Q3, G + E * F * Q3, bar, tx, tid, nt);
@@ -1219,7 +1290,7 @@ __global__ void __launch_bounds__(BK5Cfg<Eng, Q, EB, F, LAYOUT, DPAR>::NT, BK5Cf
     };
     auto issue_u = [&](long long bt) {
         const long long e0 = bt * EB;
-        const int ne = int((E - e0) < EB ? (E - e0) : EB);
+        const int ne = batch_elems<EB, S>(E, e0);
         uint32_t tx = 0;
         if (tid == 0) fence_proxy_async();
         us = stage_issue<S>(smem, u + e0 * Q3, ne * Q3, u + E * Q3, bar, tx, tid, nt);
@@ -1230,11 +1301,10 @@ __global__ void __launch_bounds__(BK5Cfg<Eng, Q, EB, F, LAYOUT, DPAR>::NT, BK5Cf
         issue_u(blockIdx.x);
     }
     uint32_t phase = 0;
-    for (long long bt = blockIdx.x; bt < nbatch; bt += gridDim.x, phase ^= 1u) {
-        if (batch_wait_failed(bar, phase, ctx, tid)) return;
+    for (long long bt = blockIdx.x < nbatch ? blockIdx.x : -1; bt >= 0; bt = walk.next, phase ^= 1u) {
+        if (walk.start(phase, ctx, tid)) return;
         const long long e0 = bt * EB;
-        const int ne = int((E - e0) < EB ? (E - e0) : EB);
-        const long long next = bt + gridDim.x;
+        const int ne = batch_elems<EB, S>(E, e0);
         const S* mb = (mass != nullptr) ? mass + e0 * Q3 : nullptr;
         const S* ub = us;
         const GS* gb = gs;
@@ -1242,18 +1312,21 @@ __global__ void __launch_bounds__(BK5Cfg<Eng, Q, EB, F, LAYOUT, DPAR>::NT, BK5Cf
         // unless the mass term reads u in the last pass (then u follows the
         // batch)
         auto early = [&]() {
-            if (next < nbatch) {
-                issue_g(next);
-                if (mass == nullptr) issue_u(next);
+            if (walk.advance(bt, phase, ctx, tid)) return true;
+            if (walk.next >= 0) {
+                issue_g(walk.next);
+                if (mass == nullptr) issue_u(walk.next);
             }
+            return false;
         };
         // the next batch's wait ends with a block barrier before anything
         // writes the boxes or the stage again, except the copy of u that
         // follows a batch with the mass term (its last pass reads u): only
         // that batch ends with its own barrier
-        bk5_sweep_batch<Eng, Q, F, LAYOUT, EO, DPAR>(prm.D, prm.eo, prm.eot, ub, gb, W0, W1, W2, W3, ne, tid, nt,
-                                                     v + e0 * Q3, mb, lambda, nullptr, early, mass != nullptr);
-        if (mass != nullptr && next < nbatch) issue_u(next);
+        if (bk5_sweep_batch<Eng, Q, F, LAYOUT, EO, DPAR>(prm.D, prm.eo, prm.eot, ub, gb, W0, W1, W2, W3, ne, tid, nt,
+                                                         v + e0 * Q3, mb, lambda, nullptr, early, mass != nullptr))
+            return;
+        if (mass != nullptr && walk.next >= 0) issue_u(walk.next);
     }
 }
 
@@ -1271,10 +1344,10 @@ struct BK1Cfg {
     static constexpr int U_BYTES = stage_bytes<S>(EB * Q3);   // also holds the P^3 output
     static constexpr int J_BYTES = stage_bytes<S>(EB * Q3);
     static constexpr int W_BYTES = ((2 * EB * WB::size * int(sizeof(V)) + 15) / 16) * 16;
-    static constexpr int SMEM = U_BYTES + J_BYTES + W_BYTES + 16;
+    static constexpr int SMEM = U_BYTES + J_BYTES + W_BYTES + kTailBytes;
 };
 
-template <class Eng, int Q, int EB, bool EO = false>
+template <class Eng, int Q, int EB, bool EO = false, bool DYN = false>
 __global__ void __launch_bounds__(BK1Cfg<Eng, Q, EB>::NT)
     bk1_kernel(const __grid_constant__ P13<typename Eng::C, Q> prm, const long long E,
                const typename Eng::S* __restrict__ u, const typename Eng::S* __restrict__ jxw, const int jxw_t,
@@ -1295,7 +1368,6 @@ __global__ void __launch_bounds__(BK1Cfg<Eng, Q, EB>::NT)
     unsigned char* jstage = ustage + Cfg::U_BYTES;
     V* W0 = reinterpret_cast<V*>(jstage + Cfg::J_BYTES);
     V* W1 = W0 + EB * WB::size;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(jstage + Cfg::J_BYTES + Cfg::W_BYTES);
     const int tid = threadIdx.x;
     const int nt = Cfg::NT;
     // interpolation out(p) = sum_i in(i) B(i, p): M(o=p, n=i) = B[i*Q + p]
@@ -1303,19 +1375,16 @@ __global__ void __launch_bounds__(BK1Cfg<Eng, Q, EB>::NT)
     // back: out(i) = sum_p in(p) B(i, p): M(o=i, n=p) = B[i*Q + p]
     const Mat<typename Eng::C, Q, false> Bb{prm.B};
 
-    if (tid == 0) {
-        mbar_init(bar, 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
     const long long nbatch = (E + EB - 1) / EB;
+    Walk<DYN> walk(jstage + Cfg::J_BYTES + Cfg::W_BYTES, nbatch, tid);
+    uint64_t* bar = walk.bar;
     // u and qdata of batch bt into the stage; the next batch is issued as
     // soon as the pointwise stage has read it (copies overlap the sweeps back)
     const S* us = nullptr;
     const S* js = nullptr;
     auto issue = [&](long long bt) {
         const long long e0 = bt * EB;
-        const int ne = int((E - e0) < EB ? (E - e0) : EB);
+        const int ne = batch_elems<EB, S>(E, e0);
         uint32_t tx = 0;
         if (tid == 0) fence_proxy_async();
         us = stage_issue<S>(ustage, u + e0 * P3, ne * P3, u + E * P3, bar, tx, tid, nt);
@@ -1324,10 +1393,10 @@ __global__ void __launch_bounds__(BK1Cfg<Eng, Q, EB>::NT)
     };
     if (blockIdx.x < nbatch) issue(blockIdx.x);
     uint32_t phase = 0;
-    for (long long bt = blockIdx.x; bt < nbatch; bt += gridDim.x, phase ^= 1u) {
+    for (long long bt = blockIdx.x < nbatch ? blockIdx.x : -1; bt >= 0; bt = walk.next, phase ^= 1u) {
         const long long e0 = bt * EB;
-        const int ne = int((E - e0) < EB ? (E - e0) : EB);
-        if (batch_wait_failed(bar, phase, ctx, tid)) return;
+        const int ne = batch_elems<EB, S>(E, e0);
+        if (walk.start(phase, ctx, tid)) return;
         if constexpr (EO) {   // B centro-symmetric (GLL nodes, Gauss points)
             if constexpr (kDirectIO) {
                 interp0_from_dense<Eng, WB, P, Q>(us, W1, ne, prm.bi, tid, nt);    // (Q,P,P)
@@ -1358,8 +1427,8 @@ __global__ void __launch_bounds__(BK1Cfg<Eng, Q, EB>::NT)
                 eor_line<Eng, Q, P, +1>(y, z, prm.bb);
                 line_store<WB, P>(W0, la, z);
             });
-            __syncthreads();
-            if (bt + gridDim.x < nbatch) issue(bt + gridDim.x);   // the stage is free
+            if (walk.advance(bt, phase, ctx, tid)) return;
+            if (walk.next >= 0) issue(walk.next);   // the stage is free
             sweep_eor<Eng, WB, 1, Q, Q, P, P, +1>(W0, W1, ne, prm.bb, tid, nt);   // (Q,P,P)
             __syncthreads();
             if constexpr (kDirectIO) {
@@ -1387,8 +1456,8 @@ __global__ void __launch_bounds__(BK1Cfg<Eng, Q, EB>::NT)
                 const int jx = jxw_t ? (k * Q + j) * Q + i : x;
                 W1[wi] = Eng::mul(W1[wi], Eng::load(js[e * Q3 + jx]));
             }
-            __syncthreads();
-            if (bt + gridDim.x < nbatch) issue(bt + gridDim.x);   // the stage is free
+            if (walk.advance(bt, phase, ctx, tid)) return;
+            if (walk.next >= 0) issue(walk.next);   // the stage is free
             sweep<Eng, WB, 2, Q, Q, Q, P>(W1, W0, ne, Bb, tid, nt);   // (Q,Q,P)
             __syncthreads();
             sweep<Eng, WB, 1, Q, Q, P, P>(W0, W1, ne, Bb, tid, nt);   // (Q,P,P)
@@ -1421,10 +1490,11 @@ struct BK3Cfg {
     static constexpr int G_BYTES = stage_bytes<S>(EB * 6 * Q3);
     static constexpr int K_BYTES = stage_bytes<S>(EB * Q3);
     static constexpr int W_BYTES = ((4 * EB * WB::size * int(sizeof(V)) + 15) / 16) * 16;
-    static constexpr int SMEM = U_BYTES + G_BYTES + K_BYTES + W_BYTES + 16;
+    static constexpr int SMEM = U_BYTES + G_BYTES + K_BYTES + W_BYTES + kTailBytes;
 };
 
-template <class Eng, int Q, int EB, bool EO = false, int DPAR = 0, class GS = typename Eng::S>
+template <class Eng, int Q, int EB, bool EO = false, int DPAR = 0, class GS = typename Eng::S,
+          bool DYN = false>
 __global__ void __launch_bounds__(BK3Cfg<Eng, Q, EB, DPAR>::NT)
     bk3_kernel(const __grid_constant__ P13<typename Eng::C, Q> prm, const long long E,
                const typename Eng::S* __restrict__ u, const GS* __restrict__ G,
@@ -1451,7 +1521,6 @@ __global__ void __launch_bounds__(BK3Cfg<Eng, Q, EB, DPAR>::NT)
     V* W1 = W0 + EB * WB::size;
     V* W2 = W1 + EB * WB::size;
     V* W3 = W2 + EB * WB::size;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(kstage + Cfg::K_BYTES + Cfg::W_BYTES);
     const int tid = threadIdx.x;
     const int nt = Cfg::NT;
     const Mat<typename Eng::C, Q, true> Bi{prm.B};    // M(p, i) = B[i*Q + p]
@@ -1459,12 +1528,9 @@ __global__ void __launch_bounds__(BK3Cfg<Eng, Q, EB, DPAR>::NT)
     const Mat<typename Eng::C, Q, true> Dg{prm.D};    // q(p) = sum_n u(n) D(n, p)
     const Mat<typename Eng::C, Q, false> Dtr{prm.D};  // sum_n f(n) D(p, n)
 
-    if (tid == 0) {
-        mbar_init(bar, 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
     const long long nbatch = (E + EB - 1) / EB;
+    Walk<DYN> walk(kstage + Cfg::K_BYTES + Cfg::W_BYTES, nbatch, tid);
+    uint64_t* bar = walk.bar;
     // u, G and k of batch bt into the stage (every thread; thread 0 issues
     // the TMA part and arrives).  The next batch is issued as soon as the
     // pointwise stage has read the stage, so its copies overlap the
@@ -1474,7 +1540,7 @@ __global__ void __launch_bounds__(BK3Cfg<Eng, Q, EB, DPAR>::NT)
     const S* ks = nullptr;
     auto issue = [&](long long bt) {
         const long long e0 = bt * EB;
-        const int ne = int((E - e0) < EB ? (E - e0) : EB);
+        const int ne = batch_elems<EB, S>(E, e0);
         uint32_t tx = 0;
         if (tid == 0) fence_proxy_async();
         us = stage_issue<S>(ustage, u + e0 * P3, ne * P3, u + E * P3, bar, tx, tid, nt);
@@ -1484,10 +1550,10 @@ __global__ void __launch_bounds__(BK3Cfg<Eng, Q, EB, DPAR>::NT)
     };
     if (blockIdx.x < nbatch) issue(blockIdx.x);
     uint32_t phase = 0;
-    for (long long bt = blockIdx.x; bt < nbatch; bt += gridDim.x, phase ^= 1u) {
+    for (long long bt = blockIdx.x < nbatch ? blockIdx.x : -1; bt >= 0; bt = walk.next, phase ^= 1u) {
         const long long e0 = bt * EB;
-        const int ne = int((E - e0) < EB ? (E - e0) : EB);
-        if (batch_wait_failed(bar, phase, ctx, tid)) return;
+        const int ne = batch_elems<EB, S>(E, e0);
+        if (walk.start(phase, ctx, tid)) return;
         // fluxes (k G grad u with the coefficient); written twice, with and
         // without k, so that no point carries predicated-off products
         auto fluxes = [&](auto with_k) {
@@ -1586,8 +1652,8 @@ __global__ void __launch_bounds__(BK3Cfg<Eng, Q, EB, DPAR>::NT)
                 fluxes(std::true_type{});
             else
                 fluxes(std::false_type{});
-            __syncthreads();
-            if (bt + gridDim.x < nbatch) issue(bt + gridDim.x);   // the stage is free
+            if (walk.advance(bt, phase, ctx, tid)) return;
+            if (walk.next >= 0) issue(walk.next);   // the stage is free
             if constexpr (DPAR) {
                 const int grp = tid / Cfg::LINES;
                 if (grp < 3) {
@@ -1648,8 +1714,8 @@ __global__ void __launch_bounds__(BK3Cfg<Eng, Q, EB, DPAR>::NT)
                 fluxes(std::true_type{});
             else
                 fluxes(std::false_type{});
-            __syncthreads();
-            if (bt + gridDim.x < nbatch) issue(bt + gridDim.x);   // the stage is free
+            if (walk.advance(bt, phase, ctx, tid)) return;
+            if (walk.next >= 0) issue(walk.next);   // the stage is free
             sweep<Eng, WB, 0, Q, Q, Q, Q>(W0, W0, ne, Dtr, tid, nt);
             sweep<Eng, WB, 1, Q, Q, Q, Q>(W1, W1, ne, Dtr, tid, nt);
             __syncthreads();

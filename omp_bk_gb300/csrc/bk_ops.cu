@@ -3,6 +3,8 @@
 // 2 fp32, 3 mixed): the build compiles this file once per engine so that the
 // translation units build in parallel.  Run-time order p -> compile-time Q
 // (the role of bk::with_order, include/bk_common.h:148-178).
+#include <type_traits>
+
 #include <cuda_runtime.h>
 
 #include "bk_internal.h"
@@ -129,6 +131,32 @@ int grid_for(long long nbatch, int occ)
     return static_cast<int>(nbatch < cap ? nbatch : cap);
 }
 
+// Launches of this many batches per resident block or more walk dynamically
+// (Walk<true>, a block per batch in the grid), smaller ones are dealt.  Times
+// dealt / dynamic: BK5 p=4 float-float at 2, 4, 8, 16 waves 18.7 / 20.5, 35.1 /
+// 37.0, 64.8 / 64.3, 125 / 120 us; BK3 p=5 FP32 at 4, 8, 15 waves 24.8 / 23.2,
+// 45.4 / 45.2, 85.7 / 82.1.
+constexpr int kDynWaves = 8;
+
+// One launch of a batch kernel: dealt (sk) or dynamic (dk) by the batches per
+// resident block, with `smem` bytes.  EB elements a batch; args: the kernel's.
+template <class Tag, bool DYN>
+struct WalkTag {};
+template <class Cfg, bool EO, int EB, class K, class... Args>
+int launch_walk(K sk, K dk, long long E, cudaStream_t s, const Args&... args)
+{
+    const long long nbatch = (E + EB - 1) / EB;
+    const int occ = prepare<WalkTag<EoTag<Cfg, EO>, false>>(sk, Cfg::SMEM, Cfg::NT);
+    if (occ <= 0) return BK_ERR_CUDA;
+    if (sk != dk && nbatch >= static_cast<long long>(kDynWaves) * occ * sm_count() && nbatch <= 0x7fffffffLL) {
+        if (prepare<WalkTag<EoTag<Cfg, EO>, true>>(dk, Cfg::SMEM, Cfg::NT) <= 0) return BK_ERR_CUDA;
+        dk<<<static_cast<int>(nbatch), Cfg::NT, Cfg::SMEM, s>>>(args..., dev_ctx());
+    } else {
+        sk<<<grid_for(nbatch, occ), Cfg::NT, Cfg::SMEM, s>>>(args..., dev_ctx());
+    }
+    return cudaGetLastError() == cudaSuccess ? BK_OK : BK_ERR_CUDA;
+}
+
 #if BK_OP_TU == 5
 // One launch of bk5_kernel with the given shape.
 // GS: the type G is stored in (the storage type, or ff2 pairs split ahead of
@@ -140,13 +168,11 @@ int bk5_launch(const P5<typename Eng::C, Q>& prm, long long E, const void* u, co
     using Cfg = BK5Cfg<Eng, Q, EB, F, LAYOUT, DPAR>;
     using S = typename Eng::S;
     static_assert(Cfg::SMEM <= 232448, "BK5 block exceeds the shared memory of an SM");
-    auto kern = bk5_kernel<Eng, Q, EB, F, LAYOUT, EO, DPAR, GS>;
-    const int occ = prepare<EoTag<Cfg, EO>>(kern, Cfg::SMEM, Cfg::NT);
-    if (occ <= 0) return BK_ERR_CUDA;
-    const int grid = grid_for((E + EB - 1) / EB, occ);
-    kern<<<grid, Cfg::NT, Cfg::SMEM, s>>>(prm, E, static_cast<const S*>(u), static_cast<const GS*>(G),
-                                          static_cast<const S*>(mass), lambda, static_cast<S*>(v), dev_ctx());
-    return cudaGetLastError() == cudaSuccess ? BK_OK : BK_ERR_CUDA;
+    // dynamic for the even-odd kernels
+    return launch_walk<Cfg, EO, EB>(&bk5_kernel<Eng, Q, EB, F, LAYOUT, EO, DPAR, GS, false>,
+                                    &bk5_kernel<Eng, Q, EB, F, LAYOUT, EO, DPAR, GS, EO>, E, s, prm, E,
+                                    static_cast<const S*>(u), static_cast<const GS*>(G), static_cast<const S*>(mass),
+                                    lambda, static_cast<S*>(v));
 }
 
 // the largest EB <= EB0 whose block fits an SM's shared memory
@@ -248,13 +274,13 @@ int bk1_q(const double* B, long long E, const void* jxw, const void* u, void* v,
     // Gauss points)
     const bool eo = make_eor<typename Eng::C, Q, Q - 1>(B, Q, true, +1, prm.bi, &Eng::coef) &&
                     make_eor<typename Eng::C, Q - 1, Q>(B, Q, false, +1, prm.bb, &Eng::coef);
-    auto kern = eo ? bk1_kernel<Eng, Q, EB, true> : bk1_kernel<Eng, Q, EB, false>;
-    const int occ = eo ? prepare<EoTag<Cfg, true>>(kern, Cfg::SMEM, Cfg::NT) : prepare<Cfg>(kern, Cfg::SMEM, Cfg::NT);
-    if (occ <= 0) return BK_ERR_CUDA;
-    const int grid = grid_for((E + EB - 1) / EB, occ);
-    kern<<<grid, Cfg::NT, Cfg::SMEM, s>>>(prm, E, static_cast<const S*>(u), static_cast<const S*>(jxw), jxw_t,
-                                          static_cast<S*>(v), dev_ctx());
-    return cudaGetLastError() == cudaSuccess ? BK_OK : BK_ERR_CUDA;
+    auto go = [&](auto e) {
+        constexpr bool EO = decltype(e)::value;
+        return launch_walk<Cfg, EO, EB>(&bk1_kernel<Eng, Q, EB, EO, false>, &bk1_kernel<Eng, Q, EB, EO, EO>, E, s, prm, E,
+                                        static_cast<const S*>(u), static_cast<const S*>(jxw), jxw_t,
+                                        static_cast<S*>(v));
+    };
+    return eo ? go(std::true_type{}) : go(std::false_type{});
 }
 
 #endif  // BK_OP_TU == 1
@@ -267,13 +293,13 @@ int bk3_launch(const P13<typename Eng::C, Q>& prm, long long E, const void* G, c
     using Cfg = BK3Cfg<Eng, Q, EB, DPAR>;
     using S = typename Eng::S;
     static_assert(Cfg::SMEM <= 232448, "BK3 block exceeds the shared memory of an SM");
-    auto kern = bk3_kernel<Eng, Q, EB, EO, DPAR, GS>;
-    const int occ = prepare<EoTag<Cfg, EO>>(kern, Cfg::SMEM, Cfg::NT);
-    if (occ <= 0) return BK_ERR_CUDA;
-    const int grid = grid_for((E + EB - 1) / EB, occ);
-    kern<<<grid, Cfg::NT, Cfg::SMEM, s>>>(prm, E, static_cast<const S*>(u), static_cast<const GS*>(G),
-                                          static_cast<const S*>(k), static_cast<S*>(v), dev_ctx());
-    return cudaGetLastError() == cudaSuccess ? BK_OK : BK_ERR_CUDA;
+    // dynamic for the even-odd kernels, but not the float-float blocks of q = 9,
+    // one to an SM, which nothing unbalances (765 us dealt against 787)
+    constexpr bool DYN = EO && !(Q == 9 && DPAR != 0);
+    return launch_walk<Cfg, EO, EB>(&bk3_kernel<Eng, Q, EB, EO, DPAR, GS, false>,
+                                    &bk3_kernel<Eng, Q, EB, EO, DPAR, GS, DYN>, E, s, prm, E,
+                                    static_cast<const S*>(u), static_cast<const GS*>(G), static_cast<const S*>(k),
+                                    static_cast<S*>(v));
 }
 
 // direction-parallel gradient stages for the float-float engine from q = 7,
@@ -281,7 +307,7 @@ int bk3_launch(const P13<typename Eng::C, Q>& prm, long long E, const void* G, c
 // 629 / 673, q = 10 763 / 1424, where a block is one element; q = 7 is level,
 // 689 / 683, and keeps the shorter latency; q = 6 loses, 614 / 592)
 constexpr bool sweep_dpar3(int q) { return eng_is_ff() && q >= 7; }
-constexpr int sweep_eb3_dpar(int q) { return q == 8 ? 2 : q == 9 ? 3 : 1; }
+constexpr int sweep_eb3_dpar(int q) { return q == 9 ? 3 : 1; }
 
 template <int Q, int EB>
 int bk3_q(const double* B, const double* D, long long E, const void* G, const void* k, const void* u, void* v,
@@ -317,14 +343,10 @@ int bk3adj_launch(const P13<typename Eng::C, Q>& prm, long long E, const void* G
     using Cfg = BK3AdjCfg<Eng, Q, EB, DPAR>;
     using S = typename Eng::S;
     static_assert(Cfg::SMEM <= 232448, "BK3 adjoint block exceeds the shared memory of an SM");
-    auto kern = bk3_adjoint_kernel<Eng, Q, EB, EO, DPAR, GS>;
-    const int occ = prepare<EoTag<Cfg, EO>>(kern, Cfg::SMEM, Cfg::NT);
-    if (occ <= 0) return BK_ERR_CUDA;
-    const int grid = grid_for((E + EB - 1) / EB, occ);
-    kern<<<grid, Cfg::NT, Cfg::SMEM, s>>>(prm, E, static_cast<const S*>(u), static_cast<const S*>(res),
-                                          static_cast<const GS*>(G), static_cast<const S*>(k), static_cast<S*>(dk),
-                                          static_cast<S*>(dG), dev_ctx());
-    return cudaGetLastError() == cudaSuccess ? BK_OK : BK_ERR_CUDA;
+    return launch_walk<Cfg, EO, EB>(&bk3_adjoint_kernel<Eng, Q, EB, EO, DPAR, GS, false>,
+                                    &bk3_adjoint_kernel<Eng, Q, EB, EO, DPAR, GS, EO>, E, s, prm, E,
+                                    static_cast<const S*>(u), static_cast<const S*>(res), static_cast<const GS*>(G),
+                                    static_cast<const S*>(k), static_cast<S*>(dk), static_cast<S*>(dG));
 }
 
 // the direction-parallel gradient sweeps for the float-float engine (q = 6

@@ -526,3 +526,38 @@ def test_apply_runs_on_the_current_stream(bklib):
         bklib.bk1_apply(p, E, B, gq, gu, v)
     s.synchronize()
     assert oracle.rel_maxdiff(host(v), ref) < TOL64
+
+
+@pytest.mark.parametrize("bk", [1, 3, 5])
+@pytest.mark.parametrize("p", P_ALL)
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_every_batch_is_taken_once(bklib, bk, p, prec):
+    """The blocks of a launch take over the batches of blocks not launched yet:
+    a launch of many waves equals the same elements in launches of one wave
+    or less, to the bit (the last batch partial, the outputs poisoned)."""
+    Q, P = (p + 1, p + 1) if bk == 5 else (p + 2, p + 1)
+    E = 40000 * 8 // Q ** 3 * 5 + 11
+    pr, dt = (bklib.PREC_FP64, torch.float64) if prec == "fp64" else (bklib.PREC_MIXED, torch.float32)
+    gen = torch.Generator(device="cuda").manual_seed(10 * bk + p)
+    u = torch.rand(E, P ** 3, generator=gen, device="cuda", dtype=torch.float64).sub_(0.5).to(dt)
+    g = torch.rand(E, (1 if bk == 1 else 6) * Q ** 3, generator=gen, device="cuda", dtype=torch.float64).to(dt)
+    D5 = bklib.bk5_matrices(p)[0]
+    B, D = bklib.bk1_bk3_matrices(p)[:2]
+
+    def apply(e0, e1):
+        gg, uu = g[e0:e1].clone(), u[e0:e1].clone()   # (an allocation of its own is aligned)
+        v = torch.full_like(uu, float("nan"))
+        if bk == 1:
+            bklib.bk1_apply(p, e1 - e0, B, gg, uu, v, prec=pr)
+        elif bk == 3:
+            bklib.bk3_apply(p, e1 - e0, B, D, gg, uu, v, prec=pr)
+        else:
+            bklib.bk5_apply(p, e1 - e0, D5, gg, uu, v, prec=pr)
+        return v
+
+    whole = apply(0, E)
+    step = max(1, min(E, 600))
+    for e0 in range(0, E, step * 7):   # a seventh of the pieces, and the last
+        assert torch.equal(whole[e0:min(E, e0 + step)], apply(e0, min(E, e0 + step)))
+    assert torch.equal(whole[max(0, E - step):], apply(max(0, E - step), E))
+    assert not torch.isnan(whole).any()
