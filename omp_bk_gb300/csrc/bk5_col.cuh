@@ -86,6 +86,49 @@ struct BK5ColCfg {
     static constexpr int SMEM = NBUF * STAGE + 3 * COL_BYTES + D_BYTES + GT_BYTES + 16 * NBUF;
 };
 
+// A column's Q values of v or the mass in global memory: with VEC (every column
+// starts on 16 or 8 bytes: the array does, and a column is a whole number of
+// such units) as 128- or 64-bit accesses; value by value a warp's access takes
+// Q times the sectors, Q values apart (mixed p=3 with the mass term, E = 125003,
+// 53.7 -> 49.4 us; the mass loaded ahead included).
+template <class S, int Q, bool VEC>
+struct GlobalCol {
+    static constexpr int B = Q * int(sizeof(S));
+    static constexpr bool kVec = VEC && B % 8 == 0 && sizeof(S) < (B % 16 == 0 ? 16 : 8);
+    using T = typename std::conditional<B % 16 == 0, float4, float2>::type;
+    static constexpr int N = int(sizeof(T) / sizeof(S));
+    __device__ static __forceinline__ void load(const S* p, S (&x)[Q])
+    {
+        if constexpr (kVec) {
+#pragma unroll
+            for (int c = 0; c < Q / N; ++c) {
+                alignas(16) S t[N];
+                *reinterpret_cast<T*>(t) = __ldcs(reinterpret_cast<const T*>(p) + c);
+#pragma unroll
+                for (int n = 0; n < N; ++n) x[c * N + n] = t[n];
+            }
+        } else {
+#pragma unroll
+            for (int n = 0; n < Q; ++n) x[n] = p[n];
+        }
+    }
+    __device__ static __forceinline__ void store(S* p, const S (&x)[Q])
+    {
+        if constexpr (kVec) {
+#pragma unroll
+            for (int c = 0; c < Q / N; ++c) {
+                alignas(16) S t[N];
+#pragma unroll
+                for (int n = 0; n < N; ++n) t[n] = x[c * N + n];
+                reinterpret_cast<T*>(p)[c] = *reinterpret_cast<const T*>(t);
+            }
+        } else {
+#pragma unroll
+            for (int n = 0; n < Q; ++n) p[n] = x[n];
+        }
+    }
+};
+
 // One batch of ne elements of order Q whose u (ub) and G (gb, in LAYOUT) are
 // staged densely in shared memory (with GDIR, gb is the batch's G in global
 // memory, column layout).  Dp: the Q x Q matrix D(i, n) in parameter
@@ -94,8 +137,10 @@ struct BK5ColCfg {
 // values; GT: the column-order G buffer (LAYOUT != 2).  vb, mb: v and the
 // optional mass at the batch's first element in global memory.  after_s2()
 // runs (by every thread) right after the second barrier, once the staged data
-// are no longer read.
-template <class Eng, int Q, int F, int LAYOUT, bool GDIR, class AfterS2>
+// are no longer read.  VEC: vb and mb start on 16 bytes, whole columns move as
+// vector accesses and the mass is loaded with G, ahead of the derivatives
+// (GlobalCol; for the FP32-storage forms).
+template <class Eng, int Q, int F, int LAYOUT, bool GDIR, bool VEC = false, class AfterS2>
 __device__ __forceinline__ void bk5_col_batch(const typename Eng::C* __restrict__ Dp, const typename Eng::V* Ds,
                                               const typename Eng::S* ub, const typename Eng::S* gb,
                                               typename Eng::V* UV, typename Eng::V* R0, typename Eng::V* R1,
@@ -131,6 +176,11 @@ __device__ __forceinline__ void bk5_col_batch(const typename Eng::C* __restrict_
 #pragma unroll
                 for (int k = 0; k < Q; ++k) gcol[f][k] = __ldcs(g0 + (f * Q + k) * Q2);
         }
+    }
+    constexpr bool kEarlyMass = VEC && GDIR;
+    S mcol[kEarlyMass ? Q : 1];
+    if constexpr (kEarlyMass) {
+        if (active && mb != nullptr) GlobalCol<S, Q, VEC>::load(mb + el * Q3 + c * Q, mcol);
     }
 
     // u of the batch -> padded columns (converted); consecutive threads read
@@ -236,7 +286,7 @@ __device__ __forceinline__ void bk5_col_batch(const typename Eng::C* __restrict_
 #pragma unroll
             for (int k = 0; k < Q; ++k) Eng::vmadd(ay[k], dy, row[k]);
         }
-        S* vo = vb + el * Q3 + c * Q;
+        S vcol[Q];
         const S* mo = (mb != nullptr) ? mb + el * Q3 + c * Q : nullptr;
 #pragma unroll
         for (int k = 0; k < Q; ++k) {
@@ -255,13 +305,16 @@ __device__ __forceinline__ void bk5_col_batch(const typename Eng::C* __restrict_
                 // + lambda * mass * u at the point
                 A am = Eng::zero();
                 Eng::add(am, res);
-                V m = Eng::load(mo[k]);
+                V m;
+                if constexpr (kEarlyMass) m = Eng::load(mcol[k]);
+                else m = Eng::load(mo[k]);
                 if (lam_scaled) m = Eng::mul(lam, m);
                 Eng::vmadd(am, m, ucol[k]);
                 res = Eng::loose(am);
             }
-            vo[k] = Eng::store(res);
+            vcol[k] = Eng::store(res);
         }
+        GlobalCol<S, Q, VEC>::store(vb + el * Q3 + c * Q, vcol);
     }
 }
 
@@ -340,7 +393,7 @@ __global__ void __launch_bounds__(BK5ColCfg<Eng, Q, EB, F, NBUF, LAYOUT>::NT)
         const S* ub = (sb == 0) ? us_slot0 : us_slot1;
         const S* gb = (sb == 0) ? gs_slot0 : gs_slot1;
         if constexpr (Cfg::GDIR) gb = G + e0 * F * Q3;
-        bk5_col_batch<Eng, Q, F, LAYOUT, Cfg::GDIR>(prm.D, Ds, ub, gb, UV, R0, R1, GT, ne, tid, nt, v + e0 * Q3,
+        bk5_col_batch<Eng, Q, F, LAYOUT, Cfg::GDIR, sizeof(S) == 4>(prm.D, Ds, ub, gb, UV, R0, R1, GT, ne, tid, nt, v + e0 * Q3,
                                          (mass != nullptr) ? mass + e0 * Q3 : nullptr, lambda, [&]() {
                                              const long long nb = bt + NBUF * stride;
                                              if (nb < nbatch) issue(nb, sb);

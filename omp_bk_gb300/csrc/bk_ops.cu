@@ -223,11 +223,23 @@ int bk5_sweep_q(int F, const double* D, long long E, const void* u, const void* 
 #endif  // BK_OP_TU == 5
 
 #if BK_OP_TU == 6
-// Column kernel: elements per block and stage buffers.  The FP32-storage
-// forms are HBM-bound (double buffering), the FP64 engines ALU-bound (one
-// stage, more blocks per SM).
-constexpr int col_nbuf() { return (sizeof(typename Eng::S) == 4) ? 2 : 1; }
-constexpr int col_eb(int q) { return (q * q >= 64) ? ((sizeof(typename Eng::S) == 4) ? 2 : 1) : (128 + q * q - 1) / (q * q); }
+// Column kernel: stage buffers.  With G read straight from HBM (FP32 storage,
+// column layout) only u is staged, and one buffer leaves room for more blocks
+// (q = 6 with the mass term 230 -> 224 us, q = 4 180 -> 177); the FP32-storage
+// forms of the other layouts take two, the FP64 engines, ALU-bound, one.
+constexpr bool col_gdir() { return sizeof(typename Eng::S) == 4 && BK_LAYOUT_TU == 2; }
+constexpr int col_nbuf() { return (sizeof(typename Eng::S) == 4 && !col_gdir()) ? 2 : 1; }
+// The elements per block that the option elems_per_block may name (0 or this).
+constexpr int col_eb_named(int q) { return (q * q >= 64) ? ((sizeof(typename Eng::S) == 4) ? 2 : 1) : (128 + q * q - 1) / (q * q); }
+// The elements per block: with G straight from HBM the fastest measured at
+// about 2^25 points with the mass term (us, the named number -> this): q = 3
+// 265 -> 252, q = 4 188 -> 177, q = 5 250 -> 241, q = 6 240 -> 224, q = 7 281
+// -> 265, q = 8 234 -> 210, q = 9 362 -> 318.
+constexpr int col_eb(int q)
+{
+    constexpr int t[8] = {32, 7, 4, 5, 3, 1, 1, 1};   // q = 2..9
+    return col_gdir() ? t[q - 2] : col_eb_named(q);
+}
 
 template <int Q, int EB, int F, int LAYOUT, int NBUF>
 int bk5col_q(const double* D, long long E, const void* u, const void* G, const void* mass, double lambda, void* v,
@@ -253,7 +265,7 @@ int bk5col_f(int F, int eb, const double* D, long long E, const void* u, const v
 {
     constexpr int NB = col_nbuf();
     constexpr int EB0 = col_eb(Q);
-    if (eb != 0 && eb != EB0) return BK_ERR_ARG;
+    if (eb != 0 && eb != col_eb_named(Q)) return BK_ERR_ARG;
     if (F == 6) return bk5col_q<Q, EB0, 6, BK_LAYOUT_TU, NB>(D, E, u, G, mass, lambda, v, s);
     if (F == 9) return bk5col_q<Q, EB0, 9, BK_LAYOUT_TU, NB>(D, E, u, G, mass, lambda, v, s);
     return BK_ERR_PREC;
