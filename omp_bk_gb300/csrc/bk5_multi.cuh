@@ -275,13 +275,36 @@ inline void multi_eo_smem(const MultiSeg* seg, int nseg, int& u_bytes, int& g_by
     total = multi_eo_nbuf<Eng>() * 2 * u_bytes + g_bytes + (dpar ? 4 : 3) * w_bytes + 16;
 }
 
+// batch_wait_failed for two barriers at once.
+__device__ __forceinline__ bool tile_wait_failed(uint64_t* bar, uint32_t phase, uint64_t* cbar, uint32_t cphase,
+                                                 const DevCtx& ctx, int tid)
+{
+    const bool ok = mbar_wait_bounded(bar, phase, ctx.wait_limit) && mbar_wait_bounded(cbar, cphase, ctx.wait_limit);
+    if (__syncthreads_or(ok ? 0 : 1)) {
+        if (tid == 0) set_status(ctx, BK_ERR_TIMEOUT);
+        if (!ok) {
+            mbar_wait_bounded(bar, phase, ctx.wait_limit);
+            mbar_wait_bounded(cbar, cphase, ctx.wait_limit);
+        }
+        return true;
+    }
+    return false;
+}
+
+// Shared memory that the dynamic launch needs beyond multi_eo_smem: the
+// answers' barrier and the answer.
+constexpr int kMultiDynBytes = 32;
+
 // DOT: also sum u . v over the launch, one partial per block in dot_part
 // (the CG's p . A p), from compensated per-thread sums.  DPAR = 2: the block
 // is three thread groups that run the three gradient sweeps, and then the
 // three transposed ones, at the same time (one shared code body, a fourth
 // work box), as the single-order float-float kernels do.  GST (FP32
 // storage): G staged by TMA instead of read straight from global memory; the
-// tuner picks the faster for a plan.
+// tuner picks the faster for a plan.  DYN: the grid has a block per tile and a
+// resident block takes over the tiles of blocks not launched yet (clc_request),
+// so that blocks with cheaper tiles do more of them; otherwise tiles b, b +
+// grid, ... are block b's.
 //
 // Staging, by mode:
 //   FP32, G direct:  u and mass double-buffered; right after tile t's wait
@@ -297,7 +320,7 @@ inline void multi_eo_smem(const MultiSeg* seg, int nseg, int& u_bytes, int& g_by
 //   FP64:            one buffer; the next tile's G after the pointwise stage
 //                    (bytes only), its u and mass after the last pass (the
 //                    arrival), as the single-order kernels do.
-template <class Eng, int NT, int MINB, bool DOT = false, int DPAR = 0, bool GST = false>
+template <class Eng, int NT, int MINB, bool DOT = false, int DPAR = 0, bool GST = false, bool DYN = false>
 __global__ void __launch_bounds__(NT, MINB)
     bk5_multi_eo_kernel(const __grid_constant__ PMultiEO<typename Eng::C> prm, const MultiTile* __restrict__ tiles,
                         const int ntiles, const typename Eng::S* __restrict__ u, const typename Eng::S* __restrict__ G,
@@ -311,6 +334,7 @@ __global__ void __launch_bounds__(NT, MINB)
     constexpr bool GD = NB == 2 && !GST;   // FP32, G read straight from global memory
     constexpr bool GS2 = NB == 2 && GST;   // FP32, G staged
     static_assert(NB == 2 || !GST, "FP64 storage always stages G");
+    static_assert(!DYN || !DOT, "a partial per block in a fixed order needs dealt tiles");
     extern __shared__ __align__(16) unsigned char smem[];
     // [u 0][mass 0]([u 1][mass 1]) [G] [W0][W1][W2]([W3]) [barrier per buffer]
     unsigned char* gstage = smem + NB * 2 * u_bytes;
@@ -319,13 +343,17 @@ __global__ void __launch_bounds__(NT, MINB)
     V* W2 = reinterpret_cast<V*>(reinterpret_cast<unsigned char*>(W1) + w_bytes);
     V* W3 = DPAR ? reinterpret_cast<V*>(reinterpret_cast<unsigned char*>(W2) + w_bytes) : nullptr;
     uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(W2) + (DPAR ? 2 : 1) * w_bytes);
+    uint64_t* cbar = bars + 2;                                // DYN
+    ClcAnswer* ans = reinterpret_cast<ClcAnswer*>(bars + 4);   // DYN
     const int tid = threadIdx.x;
     const int nt = blockDim.x;   // the plan's block: tiles with more lines loop
     if (tid == 0) {
         for (int b = 0; b < NB; ++b) mbar_init(&bars[b], 1);
+        if (DYN) mbar_init(cbar, 1);
         fence_mbar_init();
     }
     __syncthreads();
+    if (DYN && tid == 0) clc_request(ans, cbar);   // the second tile
     ffacc dacc = acc_zero();   // u . A u over the thread's points (DOT)
     // The stages of a tile are found from its descriptor (stage_at), so no
     // stage pointers stay live across tiles.
@@ -386,12 +414,21 @@ __global__ void __launch_bounds__(NT, MINB)
         }
     }
     int it = 0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+    int tn = 0;
+    for (int t = blockIdx.x; t < ntiles; t = tn, ++it) {
         const int b = (NB == 2) ? (it & 1) : 0;
         const uint32_t parity = (NB == 2) ? uint32_t((it >> 1) & 1) : uint32_t(it & 1);
-        const int tn = t + gridDim.x;
-        // nothing of the next tile is in flight yet: a failed wait just leaves
-        if (batch_wait_failed(&bars[b], parity, ctx, tid)) return;
+        // nothing of the next tile is in flight yet: a failed wait just leaves.
+        // DYN: with the tile's data comes the answer asked for during the
+        // tile before, the index of the next one (ntiles: none)
+        if constexpr (DYN) {
+            if (tile_wait_failed(&bars[b], parity, cbar, uint32_t(it & 1), ctx, tid)) return;
+            const long long a = clc_next(ans);
+            tn = a >= 0 ? int(a) : ntiles;
+        } else {
+            if (batch_wait_failed(&bars[b], parity, ctx, tid)) return;
+            tn = t + gridDim.x;
+        }
         if constexpr (NB == 2) {
             // the other buffer was last read by the previous tile, whose last
             // pass every thread finished before the wait's barrier: the next
@@ -414,6 +451,7 @@ __global__ void __launch_bounds__(NT, MINB)
         // after the pointwise stage the G stage is free for the next tile's G
         auto early = [&]() {
             __syncthreads();
+            if (DYN && tid == 0 && tn < ntiles) clc_request(ans, cbar);
             if constexpr (!GD) {
                 if (tn < ntiles) issue_g(tn, NB == 2 ? (b ^ 1) : 0, NB == 2);
             }

@@ -33,6 +33,7 @@
 namespace bkg {
 namespace {
 
+constexpr int kDynWaves = 8;   // tiles per resident block from which a launch shares them dynamically
 constexpr int kNT = 256;   // threads per block of the persistent kernel (per thread group), at most
 constexpr int kDefThreads = 128;  // threads of the sweep launch (per group) unless the plan sets them
 constexpr int kMaxTileLines = 1024;   // lines (elements x q^2) of a tile, at most
@@ -119,6 +120,10 @@ struct MultiLaunch {
 // MINB blocks per SM asked of the register allocator.  GST: FP32 G staged.
 template <class Eng, int MAXT, int MINB, bool DOT = false, int DPAR = 0, bool GST = false>
 struct MultiEOLaunch {
+    // whether large launches share their tiles dynamically: not with the fused
+    // dot product (its partials are summed in a fixed order), nor in the forms
+    // that only a tuned plan or the DFMA engine takes
+    static constexpr bool kDyn = !DOT && !GST && Eng::kId != BK_ENGINE_DFMA;
     static int threads(const MultiSeg* seg, int nseg, int block)
     {
         int nt = 64;
@@ -186,6 +191,26 @@ struct MultiEOLaunch {
         const int occ = prepare(total, nt);
         if (occ < 1) return BK_ERR_CUDA;
         int grid = occ * sm_count();
+        // from kDynWaves tiles per resident block on the blocks share the
+        // tiles dynamically (p = 2..8, 43.5 M points: mixed 340 -> 314 us,
+        // float-float 1550 -> 1507)
+        if constexpr (kDyn) {
+            if (ntiles >= kDynWaves * grid && total + kMultiDynBytes <= 232448) {
+                auto dyn = bk5_multi_eo_kernel<Eng, MAXT, MINB, false, DPAR, GST, true>;
+                static int set[kMaxDevices] = {0};
+                const int dev = current_device();
+                if (!set[dev]) {
+                    if (cudaFuncSetAttribute(dyn, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448) != cudaSuccess)
+                        return BK_ERR_CUDA;
+                    set[dev] = 1;
+                }
+                dyn<<<ntiles, nt, total + kMultiDynBytes, s>>>(prm, tiles, ntiles, static_cast<const S*>(u),
+                                                               static_cast<const S*>(G), static_cast<const S*>(mass),
+                                                               lambda, static_cast<S*>(v), ub, gb, wb, nullptr,
+                                                               dev_ctx());
+                return cudaGetLastError() == cudaSuccess ? BK_OK : BK_ERR_CUDA;
+            }
+        }
         if (grid > ntiles) grid = ntiles;
         if (grid > kMaxDotParts) grid = kMaxDotParts;
         if (nparts) *nparts = grid;
