@@ -296,7 +296,8 @@ __device__ __forceinline__ bool tile_wait_failed(uint64_t* bar, uint32_t phase, 
 constexpr int kMultiDynBytes = 32;
 
 // DOT: also sum u . v over the launch, one partial per block in dot_part
-// (the CG's p . A p), from compensated per-thread sums.  DPAR = 2: the block
+// (the CG's p . A p), from compensated per-thread sums; nothing is done if
+// *skip is not 0 (skip may be NULL).  DPAR = 2: the block
 // is three thread groups that run the three gradient sweeps, and then the
 // three transposed ones, at the same time (one shared code body, a fourth
 // work box), as the single-order float-float kernels do.  GST (FP32
@@ -326,8 +327,11 @@ __global__ void __launch_bounds__(NT, MINB)
                         const int ntiles, const typename Eng::S* __restrict__ u, const typename Eng::S* __restrict__ G,
                         const typename Eng::S* __restrict__ mass, const double lambda,
                         typename Eng::S* __restrict__ v, const int u_bytes, const int g_bytes, const int w_bytes,
-                        double* __restrict__ dot_part, const DevCtx ctx)
+                        double* __restrict__ dot_part, const double* __restrict__ skip, const DevCtx ctx)
 {
+    if constexpr (DOT) {
+        if (skip != nullptr && *skip != 0.0) return;   // (uniform)
+    }
     using S = typename Eng::S;
     using V = typename Eng::V;
     constexpr int NB = multi_eo_nbuf<Eng>();

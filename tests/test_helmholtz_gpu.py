@@ -398,3 +398,29 @@ def test_cg_preconditioners(bklib, small_plan):
         assert float(torch.linalg.norm(x - ustar) / torch.linalg.norm(ustar)) < 1e-6
         its[pc] = st["inner"]
     assert its[PRECOND_JACOBI] > 0 and its[PRECOND_NONE] > 0
+
+
+@pytest.mark.parametrize("max_inner", [1, 3, 4, 5, 8, 9])
+def test_cg_inner_limit(bklib, small_plan, max_inner):
+    """The inner CG makes the iterations asked for, also where they end inside
+    a turn of its loop: the count, and an iterate that equals that of the plan
+    with the column kernel (FP32 round-off of at most 9 iterations against
+    steps of the size of the solution: 1e-3)."""
+    bk = bklib
+    plan, G, M, ustar = small_plan
+    f = torch.empty_like(ustar)
+    plan.apply(G, M, 1.0, ustar, f, prec=bk.PREC_FP64)
+    G32, M32 = G.float(), M.float()
+    xs = []
+    try:
+        for kern in (bk.KERNEL_SWEEP, bk.KERNEL_COLUMN):
+            plan.set_kernel(kern)
+            x = torch.zeros_like(ustar)
+            st = plan.cg(G, M, G32, M32, 1.0, f, x, rtol=1e-14, max_outer=1, inner_rtol=1e-12, max_inner=max_inner,
+                         allow_noconv=True)
+            torch.cuda.synchronize()
+            assert st["inner"] == max_inner and st["outer"] == 1, st
+            xs.append(x)
+    finally:
+        plan.set_kernel(bk.KERNEL_AUTO)
+    assert float(torch.linalg.norm(xs[0] - xs[1]) / torch.linalg.norm(xs[1])) < 1e-3
