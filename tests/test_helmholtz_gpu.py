@@ -400,6 +400,36 @@ def test_cg_preconditioners(bklib, small_plan):
     assert its[PRECOND_JACOBI] > 0 and its[PRECOND_NONE] > 0
 
 
+@pytest.mark.parametrize("prec", ["ff", "mixed", "fp32"])
+def test_multi_apply_shares_tiles(bklib, prec):
+    """A launch with so many tiles that its blocks share them dynamically
+    (more than 8 for each of the 16 blocks of 128 threads an SM can hold):
+    every tile computed, eagerly and replayed from a captured graph."""
+    from omp_bk_gb300.helmholtz import HelmholtzPlan
+    plan = HelmholtzPlan([(2, 12001, 1), (3, 7003, 1), (5, 1501, 1), (8, 301, 1)])
+    try:
+        assert plan.ntiles >= 8 * 16 * 152
+        G, M = plan.geometry(seed=21)
+        u = bklib.fill_uniform(torch.empty(plan.n, dtype=torch.float64, device="cuda"), 22)
+        _check_per_order(bklib, plan, G, M, u, prec)
+        pr, dt = {"ff": (bklib.PREC_FP64, torch.float64), "mixed": (bklib.PREC_MIXED, torch.float32),
+                  "fp32": (bklib.PREC_FP32, torch.float32)}[prec]
+        Gd, Md, ud = G.to(dt), M.to(dt), u.to(dt)
+        v, w = torch.full_like(ud, float("nan")), torch.full_like(ud, float("nan"))
+        plan.apply(Gd, Md, 1.0, ud, v, prec=pr)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            plan.apply(Gd, Md, 1.0, ud, w, prec=pr)
+        for _ in range(2):
+            w.fill_(float("nan"))
+            g.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(v, w)
+    finally:
+        plan.close()
+
+
 @pytest.mark.parametrize("max_inner", [1, 3, 4, 5, 8, 9])
 def test_cg_inner_limit(bklib, small_plan, max_inner):
     """The inner CG makes the iterations asked for, also where they end inside

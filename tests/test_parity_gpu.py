@@ -561,3 +561,25 @@ def test_every_batch_is_taken_once(bklib, bk, p, prec):
         assert torch.equal(whole[e0:min(E, e0 + step)], apply(e0, min(E, e0 + step)))
     assert torch.equal(whole[max(0, E - step):], apply(max(0, E - step), E))
     assert not torch.isnan(whole).any()
+
+
+@pytest.mark.parametrize("p", P_ALL)
+@pytest.mark.parametrize("nfactors", [6, 9])
+@pytest.mark.parametrize("many", [False, True])
+def test_bk5_column_vectors(bklib, p, nfactors, many):
+    """The column kernel with G in the column layout and FP32 storage, where
+    whole columns of v and the mass move as vectors: one element, and several
+    batches per block with the last one partial, against the oracle."""
+    nq = p + 1
+    E = 320000 // nq ** 2 + 3 if many else 1
+    nq, _, dbasis, g6i, u = random_case(5, p, E)
+    G = oracle.make_bk5_G(g6i, E, nq, nfactors, bklib.LAYOUT_COLUMN)
+    mass = np.random.default_rng(p).uniform(0.5, 1.5, E * nq ** 3)
+    f = lambda a: a.astype(np.float32).astype(np.float64)
+    ref = oracle.bk5(nq, E, dbasis, f(g6i), f(u), mass=f(mass), lam=0.75)
+    gu, gg, gm = dev(u, "f32"), dev(G, "f32"), dev(mass, "f32")
+    out = torch.full_like(gu, float("nan"))
+    bklib.bk5_apply(p, E, dbasis, gg, gu, out, prec=bklib.PREC_MIXED, layout=bklib.LAYOUT_COLUMN, nfactors=nfactors,
+                    kernel=bklib.KERNEL_COLUMN, mass=gm, lam=0.75)
+    torch.cuda.synchronize()
+    assert oracle.rel_maxdiff(host(out), ref) < TOL32
