@@ -74,9 +74,10 @@ int bk_hplan_set_shape(bk_hplan_t plan, int threads, int gstage);
  * this after it.  BK_ERR_ARG for sizes out of range. */
 int bk_hplan_set_fp64_shape(bk_hplan_t plan, const int* elems_per_tile, int threads, bk_stream_t stream);
 
-/* v = A u for all orders in ONE persistent launch.  prec BK_PREC_FP64 (engine
- * AUTO/FF: float-float, DFMA: native), BK_PREC_MIXED or BK_PREC_FP32 (float
- * storage).  mass may be NULL (plain BK5). */
+/* v = A u for all orders in ONE persistent launch (large float-float applies of
+ * a plan at default shapes: one launch per order, which is faster there).  prec
+ * BK_PREC_FP64 (engine AUTO/FF: float-float, DFMA: native), BK_PREC_MIXED or
+ * BK_PREC_FP32 (float storage).  mass may be NULL (plain BK5). */
 int bk_hplan_apply(bk_hplan_t plan, const void* G, const void* mass, double lambda, const void* u, void* v,
                    int prec, int engine, bk_stream_t stream);
 

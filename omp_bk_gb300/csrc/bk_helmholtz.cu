@@ -42,7 +42,7 @@ constexpr int kMaxTileLines = 1024;   // lines (elements x q^2) of a tile, at mo
 // instead of 42 at p = 2 (the column body, one thread per column, takes 256),
 // in blocks of kDefThreads.  Against ceil(128 / q^2) elements in blocks of the
 // largest tile's lines, p = 2..8, 43.5 M points: mixed 414 -> 340 us,
-// float-float 2494 -> 1530.
+// float-float 2494 -> 1550.
 constexpr int kDefTile[7] = {28, 16, 5, 3, 2, 2, 1};
 constexpr int kRedBlocks = 1216;   // 8 blocks of 256 threads per SM
 constexpr int kMaxDotParts = 4864;  // blocks of the persistent launch at most (32 per SM)
@@ -617,6 +617,7 @@ struct bk_hplan {
     // NULL: the plan's tiles)
     MultiTile* tiles64;
     int ntiles64;
+    bool shaped;        // the caller named elements per tile
     long long n;        // values of a vector
     long long ng;       // values of G
     PMulti<double> p_dfma;
@@ -702,6 +703,26 @@ double conv_d(double x) { return x; }
 float conv_f(double x) { return float(x); }
 ff conv_ff(double x) { return EngFF::coef(x); }
 
+// Whether a float-float apply takes the orders' own kernels, one launch each:
+// their blocks have the shape and the registers of one order (q <= 7 one thread
+// per line, where the persistent launch's body runs direction groups at every
+// order).  From kOrderWaves tiles per resident block of the persistent launch
+// and order on, below which the ends of the launches cost more: us one launch /
+// per order, p = 2..8, 2.7 M points 119 / 131, 5.4 M 209 / 200, 10.9 M 396 / 324,
+// 43.5 M 1506 / 1067, p = 5, 6, 0.8 M 39.6 / 42.6, 1.6 M 71 / 69, 3.2 M 129 / 114.
+// At default shapes only (a shape that the caller set is the persistent
+// launch's), and where every order starts on 16 bytes, which the batch kernels'
+// staging counts on.
+constexpr int kOrderWaves = 4;
+bool per_order_ff(const bk_hplan* h)
+{
+    if (h->shaped || h->tiles64 || h->e_ff.block != 0) return false;
+    for (int s = 0; s < h->nseg; ++s)
+        if (h->seg[s].uoff % 2 != 0) return false;
+    const int occ = MultiFF::prepare(h->e_ff);
+    return occ > 0 && h->ntiles >= (long long)kOrderWaves * h->nseg * occ * sm_count();
+}
+
 int apply_plan(bk_hplan* h, int eng, const void* G, const void* mass, double lambda, const void* u, void* v,
                cudaStream_t s)
 {
@@ -710,7 +731,22 @@ int apply_plan(bk_hplan* h, int eng, const void* G, const void* mass, double lam
         const int n64 = h->tiles64 ? h->ntiles64 : h->ntiles;
         switch (eng) {
             case 0: return MultiEOLaunch<EngDfma, 256, 2>::run(h->e_dfma, t64, n64, u, G, mass, lambda, v, s);
-            case 1: return MultiFF::run(h->e_ff, t64, n64, u, G, mass, lambda, v, s);
+            case 1:
+                if (per_order_ff(h)) {
+                    for (int k = 0; k < h->nseg; ++k) {
+                        const MultiSeg& sg = h->seg[k];
+                        if (sg.E == 0) continue;
+                        const double* m = static_cast<const double*>(mass);
+                        const int rc = launch_bk5_ff(sg.q - 1, sg.E, h->p_dfma.D + multi_doff(sg.q),
+                                                     static_cast<const double*>(G) + sg.goff,
+                                                     static_cast<const double*>(u) + sg.uoff, m ? m + sg.uoff : nullptr,
+                                                     lambda, static_cast<double*>(v) + sg.uoff, 6, 2, 0,
+                                                     BK_KERNEL_SWEEP, BK_G_STORAGE, s);
+                        if (rc != BK_OK) return rc;
+                    }
+                    return BK_OK;
+                }
+                return MultiFF::run(h->e_ff, t64, n64, u, G, mass, lambda, v, s);
             case 2: return run_f32<EngF32>(h->e_f32, h->tiles, h->ntiles, u, G, mass, lambda, v, s);
             default:
                 return run_f32<EngMixed>(h->e_f32, h->tiles, h->ntiles, u, G, mass, lambda, v, s);
@@ -896,6 +932,7 @@ int bk_hplan_create(bk_hplan_t* out, int norders, const bk_order_range* orders, 
         }
         const int q = p + 1;
         int eb = orders[s].elems_per_tile;
+        if (eb > 0) h->shaped = true;
         if (eb <= 0) eb = kDefTile[p - 2];
         if (eb * q * q > kMaxTileLines || orders[s].E < 0 || !D[s]) {
             delete h;

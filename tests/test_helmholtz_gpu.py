@@ -454,3 +454,41 @@ def test_cg_inner_limit(bklib, small_plan, max_inner):
     finally:
         plan.set_kernel(bk.KERNEL_AUTO)
     assert float(torch.linalg.norm(xs[0] - xs[1]) / torch.linalg.norm(xs[1])) < 1e-3
+
+
+@pytest.mark.parametrize("mass", [True, False])
+@pytest.mark.parametrize("extra", [0, 1])
+def test_large_fp64_apply_by_orders(bklib, extra, mass):
+    """A float-float apply with so many tiles that the orders run in launches
+    of their own: the per-order apply to the bit; with an odd offset of the
+    second order (extra) the persistent launch computes it.  Eagerly and
+    replayed from a captured graph."""
+    from omp_bk_gb300.helmholtz import HelmholtzPlan
+    bk = bklib
+    plan = HelmholtzPlan([(8, 6000 + extra), (7, 12002), (3, 17)])
+    try:
+        assert plan.ntiles >= 4 * 3 * 6 * 152
+        G, M = plan.geometry(seed=31)
+        M = M if mass else None
+        u = bk.fill_uniform(torch.empty(plan.n, dtype=torch.float64, device="cuda"), 32)
+        v, w = torch.full_like(u, float("nan")), torch.full_like(u, float("nan"))
+        plan.apply(G, M, 0.5, u, v, prec=bk.PREC_FP64)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            plan.apply(G, M, 0.5, u, w, prec=bk.PREC_FP64)
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(v, w)
+        for k, p in enumerate(plan.p):
+            su, sg = _slices(plan, k)
+            D, _, _ = bk.bk5_matrices(p)
+            x = torch.full_like(u[su], float("nan"))
+            bk.bk5_apply(p, plan.E[k], D, G[sg].clone(), u[su].clone(), x, prec=bk.PREC_FP64, engine=bk.ENGINE_FF,
+                         layout=bk.LAYOUT_COLUMN, kernel=bk.KERNEL_SWEEP, mass=M[su].clone() if mass else None, lam=0.5)
+            torch.cuda.synchronize()
+            if extra == 0:
+                assert torch.equal(v[su], x)
+            assert oracle.rel_maxdiff(host(v[su]), host(x)) < 1e-12, p
+    finally:
+        plan.close()
