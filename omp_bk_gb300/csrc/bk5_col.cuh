@@ -9,7 +9,8 @@
 // elements, two block barriers: after the columns are published, and after
 // the fluxes rr, rs are published.
 //
-// Staging: u and G of a batch arrive by 1-D TMA bulk copies (cp.async.bulk,
+// Staging: u and G of a batch (u alone for FP32 storage with G in the column
+// layout, whose G goes from HBM to registers) arrive by 1-D TMA bulk copies (cp.async.bulk,
 // mbarrier with a bounded wait) into one of NBUF stage buffers; the copies of
 // batch it + NBUF are issued as soon as batch it no longer reads its stage
 // (after the second barrier), so they overlap the transposed derivatives and

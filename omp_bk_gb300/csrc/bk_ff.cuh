@@ -17,11 +17,11 @@
 // renormalised once at the end (12 flops per term instead of 15 for a
 // renormalising multiply-add).
 //
-// Conversions never touch the FP64 pipe on the fast path: split() cuts the
-// binary64 bit pattern into a truncated 24-bit hi and the remaining 29
-// mantissa bits (rounded to a float) with integer operations and one I2F;
-// join() adds the lo part to the bit pattern of hi as a count of double ulps.
-// Values outside [2^-74, 2^128) (split) or [2^-74, 2^127) (join) take a slow
+// Conversions do not need the FP64 pipe: split() cuts the binary64 bit pattern
+// into a truncated 24-bit hi and the remaining 29 mantissa bits (rounded to a
+// float) with integer operations and one I2F; join() adds the lo part to the
+// bit pattern of hi as a count of double ulps.  Kernels send every other value
+// through join_fp64() instead, on the otherwise idle pipe.  Values outside [2^-74, 2^128) (split) or [2^-74, 2^127) (join) take a slow
 // path through the FP64 pipe.
 //
 // Every operation uses the __f*_rn intrinsics, which the compiler never
@@ -364,10 +364,11 @@ __device__ __forceinline__ ff split(const double x)
 }
 
 // hi + lo rounded to the nearest double.  The pair is first renormalised
-// (it may be loose; FastTwoSum, see acc_result).  Fast path: the normalised hi has a biased float exponent 53..254; lo becomes an
-// integer count k of double ulps of hi (|k| <= 2^28) added to hi's binary64
-// pattern.  When hi is a power of two and lo points below it, the sum lies in
-// the binade below, whose ulp is half as large.
+// (it may be loose; FastTwoSum, see acc_result).  Fast path: the normalised hi
+// has a biased float exponent 53..254; lo becomes an integer count k of double
+// ulps of hi (|k| <= 2^28) added to hi's binary64 pattern.  When hi is a power
+// of two and lo points below it, the sum lies in the binade below, whose ulp is
+// half as large.
 __device__ __forceinline__ double join(const ff v)
 {
     float s, t;

@@ -14,12 +14,16 @@ constexpr int kMaxDevices = 64;
 
 int current_device();          // cudaGetDevice, or -1
 
-// BK5's built-in choice for BK_KERNEL_AUTO (measured on GB300 at about 2^24
-// DoFs, mixed form, GDoF/s sweep / column): the column kernel for the
+// BK5's built-in choice for BK_KERNEL_AUTO: the column kernel for the
 // FP32-storage engines (2: FP32, 3: mixed) with G in the column layout at
-// p <= 3 (p = 1..3: 100 / 129, 116 / 126, 167 / 174) and at p = 5 with the
-// mass term (131 / 135), the sweep kernel otherwise (p = 4 141 / 138, p = 5
-// without the mass term 147 / 144, p >= 6 by 19-83 %).
+// p <= 3 and at p = 5 with the mass term, the sweep kernel otherwise.  Measured
+// on GB300, mixed form, us sweep / column at 1 M, 4 M and 16 M points, with the
+// mass term: p = 1 11.2 / 9.9, 35.3 / 31.7, 129 / 118; p = 2 11.6 / 10.6, 36.4 /
+// 32.4, 124 / 120; p = 3 10.5 / 8.7, 30.1 / 25.3, 102 / 90; p = 4 11.0 / 10.8,
+// 29.7 / 32.6, 101 / 117; p = 5 11.2 / 10.4, 31.8 / 31.5, 107 / 112; p = 6 11.3 /
+// 11.2, 32.3 / 34.6, 105 / 126.  Without it: p = 2 10.8 / 10.3, 33.2 / 31.5, 116 /
+// 117; p = 3 9.4 / 8.4, 26.2 / 23.6, 88 / 83; p = 4 10.3 / 10.5, 27.7 / 31.0, 92 /
+// 113; p = 5 10.3 / 10.1, 28.3 / 30.3, 96 / 109.
 inline int bk5_builtin_auto(int p, int eng, int layout, bool with_mass)
 {
     return (eng >= 2 && layout == 2 && (p <= 3 || (p == 5 && with_mass))) ? BK_KERNEL_COLUMN : BK_KERNEL_SWEEP;

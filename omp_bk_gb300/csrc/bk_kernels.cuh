@@ -1,7 +1,8 @@
 // bk_kernels.cuh -- the BK1 / BK3 / BK5 operator kernels for sm_103a.
 //
-// One thread block processes a batch of EB elements at a time (grid-stride
-// over the batches).  Per batch:
+// One thread block processes a batch of EB elements at a time: its share of
+// the batches dealt over the grid, or the batches of blocks not launched yet
+// (Walk).  Per batch:
 //   1. stage: the batch's slices of u and of the geometric data (qdata or G)
 //      are contiguous in HBM (element-major E-vectors); each is copied into
 //      shared memory by one 1-D TMA bulk copy (cp.async.bulk, completion on an
@@ -25,8 +26,8 @@
 //      from the last interpolation's registers).
 // Work boxes are padded (row stride ZP, plane stride PS, element stride) per
 // Q from a model of the warps' shared-memory wavefronts (bk5_box, bk3_box);
-// BK3's FP32-storage box at Q = 8 also swizzles its rows and moves k lines
-// as 128-bit accesses (WBox3, BoxLine, line_load / line_store).
+// BK1's and BK3's FP32-storage box at Q = 8 also swizzles its rows and moves
+// k lines as 128-bit accesses (WBox3, BoxLine, line_load / line_store).
 #pragma once
 
 #include <cstdint>
