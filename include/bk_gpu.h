@@ -267,6 +267,14 @@ int bk_set_wait_limit(long long cycles);
  * the status word and the kernel returns normally. */
 int bk_test_wait_timeout(bk_stream_t stream);
 
+/* Test hook: a launch of one block per batch as the large applies make them
+ * (a resident block takes over batches of blocks not launched yet), nbatch
+ * blocks, at most four to an SM.  counts (device, two ints, added to): blocks
+ * that started, batches done.  stall != 0: the batches' copies never come; the
+ * resident blocks' waits give up after the wait limit, BK_ERR_TIMEOUT is
+ * recorded and the blocks not launched yet are cancelled. */
+int bk_test_walk(int nbatch, int stall, int* counts, bk_stream_t stream);
+
 /* Library version string. */
 const char* bk_version(void);
 

@@ -275,17 +275,22 @@ inline void multi_eo_smem(const MultiSeg* seg, int nseg, int& u_bytes, int& g_by
     total = multi_eo_nbuf<Eng>() * 2 * u_bytes + g_bytes + (dpar ? 4 : 3) * w_bytes + 16;
 }
 
-// batch_wait_failed for two barriers at once.
+// batch_wait_failed for the data's and the answers' barrier at once, under one
+// limit.  A data wait that gives up while the answers come ends the launch
+// (clc_drain).
 __device__ __forceinline__ bool tile_wait_failed(uint64_t* bar, uint32_t phase, uint64_t* cbar, uint32_t cphase,
-                                                 const DevCtx& ctx, int tid)
+                                                 ClcAnswer* ans, const DevCtx& ctx, int tid)
 {
-    const bool ok = mbar_wait_bounded(bar, phase, ctx.wait_limit) && mbar_wait_bounded(cbar, cphase, ctx.wait_limit);
+    auto both = [&]() {
+        const long long t0 = clock64();
+        return mbar_wait_since(bar, phase, t0, ctx.wait_limit) && mbar_wait_since(cbar, cphase, t0, ctx.wait_limit);
+    };
+    const bool ok = (mbar_try_wait(bar, phase) && mbar_try_wait(cbar, cphase)) || both();
     if (__syncthreads_or(ok ? 0 : 1)) {
         if (tid == 0) set_status(ctx, BK_ERR_TIMEOUT);
-        if (!ok) {
-            mbar_wait_bounded(bar, phase, ctx.wait_limit);
-            mbar_wait_bounded(cbar, cphase, ctx.wait_limit);
-        }
+        if (!ok) both();
+        if (tid == 0 && mbar_try_wait(cbar, cphase) && clc_next(ans) >= 0)
+            clc_drain(ans, cbar, cphase ^ 1u, ctx.wait_limit);
         return true;
     }
     return false;
@@ -426,7 +431,7 @@ __global__ void __launch_bounds__(NT, MINB)
         // DYN: with the tile's data comes the answer asked for during the
         // tile before, the index of the next one (ntiles: none)
         if constexpr (DYN) {
-            if (tile_wait_failed(&bars[b], parity, cbar, uint32_t(it & 1), ctx, tid)) return;
+            if (tile_wait_failed(&bars[b], parity, cbar, uint32_t(it & 1), ans, ctx, tid)) return;
             const long long a = clc_next(ans);
             tn = a >= 0 ? int(a) : ntiles;
         } else {

@@ -9,6 +9,7 @@
 #include "bk_device.cuh"
 #include "bk_gpu.h"
 #include "bk_internal.h"
+#include "bk_kernels.cuh"
 
 #define BK_VERSION "omp_bk_gb300 0.1 (sm_103a)"
 
@@ -88,6 +89,26 @@ __global__ void wait_timeout_kernel(const DevCtx ctx)
     // nothing arrives on the barrier: the bounded wait must give up
     if (!mbar_wait_bounded(&bar, 0, ctx.wait_limit)) {
         if (threadIdx.x == 0) set_status(ctx, BK_ERR_TIMEOUT);
+    }
+}
+
+// A launch with a block per batch whose batches are counted and no more; with
+// `stall` the copies' barrier is armed and nothing completes it.
+__global__ void walk_kernel(const long long nbatch, const int stall, int* counts, const DevCtx ctx)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int tid = threadIdx.x;
+    Walk<true> walk(smem, nbatch, tid);
+    if (tid == 0) atomicAdd(counts, 1);
+    uint32_t phase = 0;
+    for (long long bt = blockIdx.x; bt >= 0; bt = walk.next, phase ^= 1u) {
+        if (tid == 0) {
+            if (stall) mbar_arrive_expect_tx(walk.bar, 16);
+            else mbar_arrive(walk.bar);
+        }
+        if (walk.start(phase, ctx, tid)) return;
+        if (tid == 0) atomicAdd(counts + 1, 1);
+        if (walk.advance(bt, phase, ctx, tid)) return;
     }
 }
 
@@ -351,6 +372,17 @@ int bk_test_wait_timeout(bk_stream_t stream)
     const DevCtx c = dev_ctx();
     if (c.status == nullptr) return BK_ERR_CUDA;
     wait_timeout_kernel<<<1, 32, 0, reinterpret_cast<cudaStream_t>(stream)>>>(c);
+    return cudaGetLastError() == cudaSuccess ? BK_OK : BK_ERR_CUDA;
+}
+
+int bk_test_walk(int nbatch, int stall, int* counts, bk_stream_t stream)
+{
+    if (counts == nullptr) return BK_ERR_NULL;
+    if (nbatch < 1) return BK_ERR_SIZE;
+    const DevCtx c = dev_ctx();
+    if (c.status == nullptr) return BK_ERR_CUDA;
+    // 48 KB a block: four to an SM
+    walk_kernel<<<nbatch, 32, 49152, reinterpret_cast<cudaStream_t>(stream)>>>(nbatch, stall != 0, counts, c);
     return cudaGetLastError() == cudaSuccess ? BK_OK : BK_ERR_CUDA;
 }
 

@@ -74,6 +74,16 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity)
     return ok != 0;
 }
 
+// Waits for phase `parity` of the barrier until `limit` SM cycles after t0
+// (a clock64 value).  Returns false when it gave up.
+__device__ __forceinline__ bool mbar_wait_since(uint64_t* bar, uint32_t parity, long long t0, long long limit)
+{
+    while (!mbar_try_wait(bar, parity)) {
+        if (clock64() - t0 > limit) return false;
+    }
+    return true;
+}
+
 // Waits for phase `parity` of the barrier for at most `limit` SM cycles.
 // Returns false when it gave up.  Never spins without bound.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, long long limit)
@@ -81,13 +91,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     if (mbar_try_wait(bar, parity)) {
         return true;
     }
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity)) {
-        if (clock64() - t0 > limit) {
-            return false;
-        }
-    }
-    return true;
+    return mbar_wait_since(bar, parity, clock64(), limit);
 }
 
 // ---- 1-D TMA bulk copies -----------------------------------------------------
@@ -162,6 +166,24 @@ __device__ __forceinline__ long long clc_next(const ClcAnswer* a)
         : "r"(smem_u32(a))
         : "memory");
     return ok ? static_cast<long long>(x) : -1;
+}
+
+// The end of a launch with a block per batch, one of whose blocks gave up a
+// wait for its data (one thread of that block, no request open): takes over
+// every block not launched yet and does nothing for it.  Without it each of
+// them would be launched in turn to wait out its own limit, hours for a launch
+// of many waves.  parity: of `bar`'s current phase.  (Inline: as a call it cost
+// the kernels registers, and the mixed-order one spills, 314 -> 454 us.)
+__device__ __forceinline__ void clc_drain(ClcAnswer* a, uint64_t* bar, uint32_t parity, long long limit)
+{
+    do {
+        clc_request(a, bar);
+        if (!mbar_wait_bounded(bar, parity, limit)) {
+            mbar_wait_bounded(bar, parity, limit);   // the answer may still land
+            return;
+        }
+        parity ^= 1u;
+    } while (clc_next(a) >= 0);
 }
 
 // One arrival on the barrier (no transaction bytes).

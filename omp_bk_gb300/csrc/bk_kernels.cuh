@@ -801,6 +801,9 @@ __device__ __forceinline__ int batch_elems(long long E, long long e0)
 //     launches of a few waves, where the answers' latency shows.
 // A template parameter and not a flag of the launch: with a flag the compiler
 // kept more registers over the batch (adjoint p=4 729 -> 766 us).
+// Waits: a block whose data does not come gives up after the limit and ends the
+// launch with it (clc_drain), so that the launch is over after about two limits
+// however many batches it has.  An answer is waited for under the limit too.
 // The tail of a block's shared memory: the data barrier, the walk's, and its
 // answer.
 constexpr int kTailBytes = 32;
@@ -823,10 +826,14 @@ struct Walk {
         }
         __syncthreads();
     }
-    // waits for the batch's copies; true on a timeout (batch_wait_failed)
+    // waits for the batch's copies; true on a timeout (batch_wait_failed),
+    // after which the batches of blocks not launched yet are given up too
     __device__ __forceinline__ bool start(uint32_t phase, const DevCtx& ctx, int tid) const
     {
-        if (batch_wait_failed(bar, phase, ctx, tid)) return true;
+        if (batch_wait_failed(bar, phase, ctx, tid)) {
+            if (DYN && tid == 0) clc_drain(ans, cbar, phase, ctx.wait_limit);
+            return true;
+        }
         if (DYN && tid == 0) clc_request(ans, cbar);
         return false;
     }

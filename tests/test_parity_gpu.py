@@ -583,3 +583,47 @@ def test_bk5_column_vectors(bklib, p, nfactors, many):
                     kernel=bklib.KERNEL_COLUMN, mass=gm, lam=0.75)
     torch.cuda.synchronize()
     assert oracle.rel_maxdiff(host(out), ref) < TOL32
+
+
+def test_stalled_launch_ends_after_one_limit(bklib):
+    """A launch with a block per batch whose copies never come ends after the
+    waits of its first resident blocks: the others are cancelled.  The status
+    that it leaves stops no later launch, nor a replay of a captured one, before
+    the host clears it."""
+    L = bklib.lib()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    nbatch = 64 * 4 * sms   # 64 rounds of the resident blocks, four to an SM
+    few = 8 * sms           # those, and the ones launched while the first give up
+    counts = torch.zeros(2, dtype=torch.int32, device="cuda")
+
+    def walk(stall):
+        counts.zero_()
+        assert L.bk_test_walk(nbatch, stall, counts.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        return counts.tolist()
+
+    assert bklib.device_status(reset=True) == bklib.BK_OK
+    started, done = walk(0)
+    assert done == nbatch and started < nbatch
+    assert L.bk_set_wait_limit(200000) == 0
+    try:
+        started, done = walk(1)
+        assert 1 <= started <= few and done == 0
+        assert bklib.device_status(reset=False) == bklib.BK_ERR_TIMEOUT
+        assert walk(0)[1] == nbatch
+        assert bklib.device_status(reset=True) == bklib.BK_ERR_TIMEOUT   # the first error stays
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            assert L.bk_test_walk(nbatch, 1, counts.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+        for _ in range(2):
+            counts.zero_()
+            g.replay()
+            torch.cuda.synchronize()
+            assert 1 <= counts[0].item() <= few and counts[1].item() == 0
+    finally:
+        assert L.bk_set_wait_limit(0) == 0
+        bklib.device_status(reset=True)
+    p, E = 3, 4
+    nq, _, dbasis, g, u = random_case(5, p, E)
+    out = gpu_apply(bklib, 5, p, E, None, dbasis, g, u, bklib.PREC_FP64)
+    assert oracle.rel_maxdiff(out, oracle.bk5(nq, E, dbasis, g, u)) < TOL64
