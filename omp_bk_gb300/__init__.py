@@ -19,6 +19,7 @@ import ctypes as C
 import functools
 import os
 from dataclasses import dataclass
+from operator import index
 
 import numpy as np
 
@@ -215,12 +216,18 @@ class ApplyOptions:
                        self.gform, self.jxw_layout)
 
 
-@functools.lru_cache(maxsize=512, typed=True)
+@functools.lru_cache(maxsize=512)
+def _options(*values: int):
+    return C.byref(Options(*values))
+
+
 def _opt(prec=PREC_FP64, engine=ENGINE_AUTO, layout=LAYOUT_INTERLEAVED, nfactors=6, elems_per_block=0,
          kernel=KERNEL_AUTO, gform=G_STORAGE, jxw_layout=JXW_PQR):
     """A reference to the bk_options of these values (read by the library
-    only, so one structure per set of values serves every call)."""
-    return C.byref(Options(prec, engine, layout, nfactors, elems_per_block, kernel, gform, jxw_layout))
+    only, so one structure per set of values serves every call).  The values
+    are read from their objects here: an array's or a tensor's may change."""
+    return _options(index(prec), index(engine), index(layout), index(nfactors), index(elems_per_block),
+                    index(kernel), index(gform), index(jxw_layout))
 
 
 # ---- operator apply (device tensors) -------------------------------------------

@@ -212,3 +212,24 @@ def test_option_values_are_kept_apart():
     assert (a._obj.prec, a._obj.layout, a._obj.nfactors) == (bk.PREC_FP32, 2, 6)
     with pytest.raises(TypeError):
         bk._opt(prec=float(bk.PREC_FP32), layout=2)
+
+
+def test_option_objects_are_read_each_call():
+    """An option may be any integer object (a numpy or torch scalar): its value
+    at the call counts, also where the same object held another one before."""
+    import torch
+
+    import omp_bk_gb300 as bk
+
+    def seen(**kw):
+        o = bk._opt(**kw)._obj
+        return o.prec, o.engine, o.layout, o.gform
+
+    t = torch.tensor(bk.PREC_FP32)
+    assert seen(prec=t)[0] == bk.PREC_FP32
+    t.fill_(bk.PREC_MIXED)
+    assert seen(prec=t)[0] == bk.PREC_MIXED
+    a = np.array(bk.LAYOUT_COLUMN)
+    assert seen(layout=a, prec=np.int64(bk.PREC_FP32), engine=np.int8(1), gform=True) == (bk.PREC_FP32, 1, 2, 1)
+    a[...] = bk.LAYOUT_FACTOR
+    assert seen(layout=a)[2] == bk.LAYOUT_FACTOR
