@@ -411,27 +411,47 @@ __global__ void __launch_bounds__(kRedThreads) cg_init_scalars_kernel(const doub
 // Scalars: every block reads the ones its kernel needs, and block 0 writes
 // only such as no block of the same kernel reads.
 
-// r -= alpha Ap at four points and their terms of r.z (z = w .* r) into t,
-// each product exact and the sum compensated (acc_madd_f)
-__device__ __forceinline__ float4 cg_update4(float alpha, const float4& aa, float4 rr, const float4& w, ffacc& t)
+// Float to double by integer operations, for normal numbers (is_normal): the
+// conversion instruction runs on the FP64 pipe, which has 1/64 of the rate.
+__device__ __forceinline__ bool is_normal(float x)
+{
+    return (__float_as_uint(x) & 0x7fffffffu) - 0x00800000u < 0x7f000000u;
+}
+__device__ __forceinline__ double widen_normal(float x)
+{
+    const uint32_t b = __float_as_uint(x);
+    // the exponent's bias 127 -> 1023; 20 + 3 bits of mantissa
+    return __hiloint2double(int((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), int(b << 29));
+}
+
+// r -= alpha Ap at four points and their terms of r.z (z = w .* r) added to s:
+// every product exact, every sum in FP64
+__device__ __forceinline__ float4 cg_update4(float alpha, const float4& aa, float4 rr, const float4& w, double& s)
 {
     rr.x = fmaf(-alpha, aa.x, rr.x);
     rr.y = fmaf(-alpha, aa.y, rr.y);
     rr.z = fmaf(-alpha, aa.z, rr.z);
     rr.w = fmaf(-alpha, aa.w, rr.w);
-    acc_madd_f(t, rr.x, __fmul_rn(w.x, rr.x));
-    acc_madd_f(t, rr.y, __fmul_rn(w.y, rr.y));
-    acc_madd_f(t, rr.z, __fmul_rn(w.z, rr.z));
-    acc_madd_f(t, rr.w, __fmul_rn(w.w, rr.w));
+    const float r[4] = {rr.x, rr.y, rr.z, rr.w};
+    const float z[4] = {w.x * rr.x, w.y * rr.y, w.z * rr.z, w.w * rr.w};
+    bool fast = true;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) fast = fast & is_normal(r[k]) & is_normal(z[k]);
+    if (fast) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s = fma(widen_normal(r[k]), widen_normal(z[k]), s);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s = fma(double(r[k]), double(z[k]), s);
+    }
     return rr;
 }
 
 // alpha = r.z / p.Ap, r -= alpha Ap and the partial sums of the new r.z =
 // r.(invd .* r) (r.r without the preconditioner, invd = 1).  part: the nb
-// partials of p.Ap; rpart: out.  The terms of eight points are summed in
-// float-float (2^-48 of their sum, which is of one sign) before they join the
-// thread's FP64 sum: with two conversions and an FP64 fma per point the FP64
-// pipe bounded the kernel (32 us of its 38 at 5.4 M points).
+// partials of p.Ap; rpart: out.  One instruction per point on the FP64 pipe,
+// the fma: with its operands' conversions there too the pipe bounded the kernel
+// (32 us of its 38 at 5.4 M points).
 __global__ void __launch_bounds__(kCgThreads) cg_update_kernel(long long n, int turn, double* __restrict__ sc,
                                                                const double* __restrict__ part, int nb,
                                                                const float* __restrict__ Ap, float* __restrict__ r,
@@ -452,22 +472,19 @@ __global__ void __launch_bounds__(kCgThreads) cg_update_kernel(long long n, int 
     const float4* w4 = reinterpret_cast<const float4*>(invd);
     float4* r4 = reinterpret_cast<float4*>(r);
     double s = 0.0;
-    for (long long i = blockIdx.x * (long long)kCgThreads + threadIdx.x; i < n4; i += 2 * stride) {
+    long long i = blockIdx.x * (long long)kCgThreads + threadIdx.x;
+    for (; i + stride < n4; i += 2 * stride) {
         const long long j = i + stride;
-        const bool two = j < n4;
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
         const float4 a0 = a4[i], r0 = r4[i], w0 = w4[i];
-        const float4 a1 = two ? a4[j] : zero, r1 = two ? r4[j] : zero, w1 = two ? w4[j] : zero;
-        ffacc t = acc_zero();
-        r4[i] = cg_update4(alpha, a0, r0, w0, t);
-        const float4 q = cg_update4(alpha, a1, r1, w1, t);
-        if (two) r4[j] = q;
-        s += double(t.s) + double(t.c);
+        const float4 a1 = a4[j], r1 = r4[j], w1 = w4[j];
+        r4[i] = cg_update4(alpha, a0, r0, w0, s);
+        r4[j] = cg_update4(alpha, a1, r1, w1, s);
     }
-    for (long long i = 4 * n4 + blockIdx.x * (long long)kCgThreads + threadIdx.x; i < n; i += stride) {
-        const float ri = fmaf(-alpha, Ap[i], r[i]);
-        r[i] = ri;
-        s = fma(double(ri), double(invd[i] * ri), s);
+    if (i < n4) r4[i] = cg_update4(alpha, a4[i], r4[i], w4[i], s);
+    for (long long k = 4 * n4 + blockIdx.x * (long long)kCgThreads + threadIdx.x; k < n; k += stride) {
+        const float rk = fmaf(-alpha, Ap[k], r[k]);
+        r[k] = rk;
+        s = fma(double(rk), double(invd[k] * rk), s);
     }
     const double t = block_reduce<kCgThreads>(s);
     if (threadIdx.x == 0) rpart[blockIdx.x] = t;

@@ -492,3 +492,31 @@ def test_large_fp64_apply_by_orders(bklib, extra, mass):
             assert oracle.rel_maxdiff(host(v[su]), host(x)) < 1e-12, p
     finally:
         plan.close()
+
+
+def test_cg_scaled_operator(bklib, small_plan):
+    """The solve of 2^80 A x = 2^80 f on the column body makes the iterations of
+    that of A x = f: every step of it scales exactly, and its dot products are
+    FP64 sums of exact products.  (The directions stay above 2^-126; the products
+    of r.z, below 2^-150 near the end, would underflow in FP32.)  The iterates may
+    differ by what single directions below 2^-126 lose: 1e-3 of the FP32 solve's
+    error, which is 1e-6 of the solution."""
+    bk = bklib
+    plan, G, M, ustar = small_plan
+    res = {}
+    try:
+        plan.set_kernel(bk.KERNEL_COLUMN)
+        for scale in (1.0, 2.0 ** 80):
+            Gs, Ms = G * scale, M * scale
+            f = torch.empty_like(ustar)
+            plan.apply(Gs, Ms, 1.0, ustar, f, prec=bk.PREC_FP64)
+            x = torch.zeros_like(ustar)
+            st = plan.cg(Gs, Ms, Gs.float(), Ms.float(), 1.0, f, x, rtol=1e-14, max_outer=1, inner_rtol=1e-9,
+                         max_inner=2000, allow_noconv=True)
+            torch.cuda.synchronize()
+            res[scale] = st["inner"], x
+    finally:
+        plan.set_kernel(bk.KERNEL_AUTO)
+    (n1, x1), (n2, x2) = res.values()
+    assert n1 == n2 and 10 < n1 < 2000
+    assert float(torch.linalg.norm(x1 - x2) / torch.linalg.norm(x1)) < 1e-9
