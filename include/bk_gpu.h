@@ -275,6 +275,10 @@ int bk_test_wait_timeout(bk_stream_t stream);
  * recorded and the blocks not launched yet are cancelled. */
 int bk_test_walk(int nbatch, int stall, int* counts, bk_stream_t stream);
 
+/* Test hook: n float-float pairs (device, 2 n floats, 8-byte aligned) as doubles
+ * by the two routes of the stores: out[0, n) integer, out[n, 2 n) FP64. */
+int bk_test_join(int64_t n, const void* pairs, double* out, bk_stream_t stream);
+
 /* Library version string. */
 const char* bk_version(void);
 

@@ -43,7 +43,7 @@ JXW_PQR, JXW_RQP = 0, 1
 EXPORTS = [
     "bk_default_options", "bk1_apply", "bk3_apply", "bk5_apply", "bk1_apply_opt", "bk3_apply_opt",
     "bk5_apply_opt", "bk5_apply_ex", "bk3_apply_k", "bk_device_status", "bk_set_wait_limit",
-    "bk_test_wait_timeout", "bk_test_walk", "bk_version",
+    "bk_test_wait_timeout", "bk_test_walk", "bk_test_join", "bk_version",
     "bk_gauss_points", "bk_gll_points", "bk_lagrange_interp", "bk_lagrange_deriv", "bk_fill_uniform",
     "bk_fill_lognormal", "bk_geom_affine", "bk_coords_affine", "bk_geom_trilinear", "bk_convert",
     "bk3_adjoint", "bk_stream_kernel", "bk_dot_workspace_bytes", "bk_dot", "bk_axpby",
@@ -98,6 +98,7 @@ def lib():
         "bk_set_wait_limit": [C.c_longlong],
         "bk_test_wait_timeout": [_vp],
         "bk_test_walk": [C.c_int, C.c_int, _vp, _vp],
+        "bk_test_join": [_i64, _vp, _vp, _vp],
         "bk_gauss_points": [C.c_int, _dp, _dp],
         "bk_gll_points": [C.c_int, _dp, _dp],
         "bk_lagrange_interp": [C.c_int, _dp, C.c_int, _dp, _dp],

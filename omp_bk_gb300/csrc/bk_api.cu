@@ -112,6 +112,15 @@ __global__ void walk_kernel(const long long nbatch, const int stall, int* counts
     }
 }
 
+__global__ void join_kernel(const long long n, const float2* __restrict__ pairs, double* __restrict__ out)
+{
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const ff v{pairs[i].x, pairs[i].y};
+        out[i] = join(v);
+        out[n + i] = join_fp64(v);
+    }
+}
+
 }  // namespace bkg
 
 using namespace bkg;
@@ -383,6 +392,14 @@ int bk_test_walk(int nbatch, int stall, int* counts, bk_stream_t stream)
     if (c.status == nullptr) return BK_ERR_CUDA;
     // 48 KB a block: four to an SM
     walk_kernel<<<nbatch, 32, 49152, reinterpret_cast<cudaStream_t>(stream)>>>(nbatch, stall != 0, counts, c);
+    return cudaGetLastError() == cudaSuccess ? BK_OK : BK_ERR_CUDA;
+}
+
+int bk_test_join(int64_t n, const void* pairs, double* out, bk_stream_t stream)
+{
+    if (pairs == nullptr || out == nullptr) return BK_ERR_NULL;
+    if (n < 1) return BK_ERR_SIZE;
+    join_kernel<<<256, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(n, static_cast<const float2*>(pairs), out);
     return cudaGetLastError() == cudaSuccess ? BK_OK : BK_ERR_CUDA;
 }
 

@@ -627,3 +627,23 @@ def test_stalled_launch_ends_after_one_limit(bklib):
     nq, _, dbasis, g, u = random_case(5, p, E)
     out = gpu_apply(bklib, 5, p, E, None, dbasis, g, u, bklib.PREC_FP64)
     assert oracle.rel_maxdiff(out, oracle.bk5(nq, E, dbasis, g, u)) < TOL64
+
+
+def test_joins_agree(bklib):
+    """A float-float pair becomes the nearest double of hi + lo by both routes of
+    the stores, whichever part is the larger: loose pairs after a cancellation,
+    normalised ones, powers of two with a part below, zeros."""
+    rng = np.random.default_rng(11)
+    n = 1 << 20
+    hi = (rng.uniform(1, 2, n) * 2.0 ** rng.integers(-30, 30, n) * rng.choice([-1, 1], n)).astype(np.float32)
+    lo = (rng.uniform(1, 2, n) * np.abs(hi) * 2.0 ** rng.integers(-50, 30, n) * rng.choice([-1, 1], n)).astype(np.float32)
+    hi[::7] = np.exp2(np.floor(np.log2(np.abs(hi[::7]))))
+    hi[::1001], lo[::1003] = 0, 0
+    hi[5], lo[5] = 2.0 ** -24, 1 + 2.0 ** -23
+    pairs = torch.from_numpy(np.stack([hi, lo], axis=1)).cuda()
+    out = torch.empty(2, n, dtype=torch.float64, device="cuda")
+    assert bklib.lib().bk_test_join(n, pairs.data_ptr(), out.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    want = hi.astype(np.float64) + lo.astype(np.float64)
+    got = out.cpu().numpy()
+    assert np.array_equal(got[1], want) and np.array_equal(got[0], want)
