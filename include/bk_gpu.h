@@ -95,10 +95,15 @@ typedef struct bk_options {
     int layout;    /* BK5: bk_layout; BK3 reads G factor-major (bk3_sumfact.h:53) */
     int nfactors;  /* BK5: 6 (symmetric rr rs rt ss st tt) or 9 (full 3x3,
                       row-major; bk5_offload.cpp "F") */
-    int elems_per_block; /* BK5 column kernel: elements per thread block, 0
-                            or its default (other values BK_ERR_ARG); the
-                            sweep kernels use per-order tables measured on
-                            GB300 and ignore it */
+    int elems_per_block; /* BK5 column kernel: elements per thread block: 0
+                            (its default), that default, or those of about
+                            128 columns, 32, 15, 8, 6, 4, 3, 2, 2 for p =
+                            1..8 (FP64 storage 1 at p = 7, 8), which is its
+                            default but for FP32 storage with G in the
+                            column layout (32, 7, 4, 5, 3, 1, 1, 1); other
+                            values BK_ERR_ARG.  The sweep kernels use
+                            per-order tables measured on GB300 and ignore
+                            it */
     int kernel;    /* bk_kernel_shape (BK5); BK1/BK3 have the sweep kernel only */
     int gform;     /* bk_gform (BK5, BK3, the adjoint): how G is stored */
     int jxw_layout; /* bk_jxw_layout (BK1): the order of qdata's points */

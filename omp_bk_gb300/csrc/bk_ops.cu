@@ -229,16 +229,16 @@ int bk5_sweep_q(int F, const double* D, long long E, const void* u, const void* 
 // forms of the other layouts take two, the FP64 engines, ALU-bound, one.
 constexpr bool col_gdir() { return sizeof(typename Eng::S) == 4 && BK_LAYOUT_TU == 2; }
 constexpr int col_nbuf() { return (sizeof(typename Eng::S) == 4 && !col_gdir()) ? 2 : 1; }
-// The elements per block that the option elems_per_block may name (0 or this).
-constexpr int col_eb_named(int q) { return (q * q >= 64) ? ((sizeof(typename Eng::S) == 4) ? 2 : 1) : (128 + q * q - 1) / (q * q); }
-// The elements per block: with G straight from HBM the fastest measured at
-// about 2^25 points with the mass term (us, the named number -> this): q = 3
-// 265 -> 252, q = 4 188 -> 177, q = 5 250 -> 241, q = 6 240 -> 224, q = 7 281
-// -> 265, q = 8 234 -> 210, q = 9 362 -> 318.
+// Elements per block: about 128 columns.
+constexpr int col_eb_128(int q) { return (q * q >= 64) ? ((sizeof(typename Eng::S) == 4) ? 2 : 1) : (128 + q * q - 1) / (q * q); }
+// The default: with G straight from HBM the fastest measured at about 2^25
+// points with the mass term (us, about 128 columns -> this): q = 3 265 -> 252,
+// q = 4 188 -> 177, q = 5 250 -> 241, q = 6 240 -> 224, q = 7 281 -> 265, q = 8
+// 234 -> 210, q = 9 362 -> 318.
 constexpr int col_eb(int q)
 {
     constexpr int t[8] = {32, 7, 4, 5, 3, 1, 1, 1};   // q = 2..9
-    return col_gdir() ? t[q - 2] : col_eb_named(q);
+    return col_gdir() ? t[q - 2] : col_eb_128(q);
 }
 
 template <int Q, int EB, int F, int LAYOUT, int NBUF>
@@ -263,11 +263,20 @@ template <int Q>
 int bk5col_f(int F, int eb, const double* D, long long E, const void* u, const void* G, const void* mass,
              double lambda, void* v, cudaStream_t s)
 {
+    // the option names the default or about 128 columns, and gets what it names
     constexpr int NB = col_nbuf();
     constexpr int EB0 = col_eb(Q);
-    if (eb != 0 && eb != col_eb_named(Q)) return BK_ERR_ARG;
-    if (F == 6) return bk5col_q<Q, EB0, 6, BK_LAYOUT_TU, NB>(D, E, u, G, mass, lambda, v, s);
-    if (F == 9) return bk5col_q<Q, EB0, 9, BK_LAYOUT_TU, NB>(D, E, u, G, mass, lambda, v, s);
+    constexpr int EB1 = col_eb_128(Q);
+    if (eb == 0) eb = EB0;
+    if (eb != EB0 && eb != EB1) return BK_ERR_ARG;
+    if (F == 6) {
+        if (eb == EB0) return bk5col_q<Q, EB0, 6, BK_LAYOUT_TU, NB>(D, E, u, G, mass, lambda, v, s);
+        return bk5col_q<Q, EB1, 6, BK_LAYOUT_TU, NB>(D, E, u, G, mass, lambda, v, s);
+    }
+    if (F == 9) {
+        if (eb == EB0) return bk5col_q<Q, EB0, 9, BK_LAYOUT_TU, NB>(D, E, u, G, mass, lambda, v, s);
+        return bk5col_q<Q, EB1, 9, BK_LAYOUT_TU, NB>(D, E, u, G, mass, lambda, v, s);
+    }
     return BK_ERR_PREC;
 }
 #endif  // BK_OP_TU == 6

@@ -647,3 +647,40 @@ def test_joins_agree(bklib):
     want = hi.astype(np.float64) + lo.astype(np.float64)
     got = out.cpu().numpy()
     assert np.array_equal(got[1], want) and np.array_equal(got[0], want)
+
+
+@pytest.mark.parametrize("p", P_ALL)
+@pytest.mark.parametrize("layout", [0, 1, 2])
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_bk5_column_elements_per_block(bklib, prec, layout, p):
+    """The column kernel's elems_per_block: 0, the documented default and about
+    128 columns are taken and give the same result (elements are independent of
+    the block they are in), every other number is refused."""
+    nq, E = p + 1, 37
+    _, _, dbasis, g6i, u = random_case(5, p, E)
+    G = oracle.make_bk5_G(g6i, E, nq, 6, layout)
+    t = "f64" if prec == "fp64" else "f32"
+    gu, gg = dev(u, t), dev(G, t)
+    pr = bklib.PREC_FP64 if prec == "fp64" else bklib.PREC_MIXED
+    allowed = {0, (32, 15, 8, 6, 4, 3, 2, 2)[p - 1] if prec == "mixed" or p < 7 else 1}
+    if prec == "mixed" and layout == bklib.LAYOUT_COLUMN:
+        allowed.add((32, 7, 4, 5, 3, 1, 1, 1)[p - 1])
+    ref = None
+    for eb in range(65):
+        out = torch.full_like(gu, float("nan"))
+
+        def run():
+            bklib.bk5_apply(p, E, dbasis, gg, gu, out, prec=pr, layout=layout, kernel=bklib.KERNEL_COLUMN,
+                            elems_per_block=eb)
+
+        if eb not in allowed:
+            with pytest.raises(bklib.BKError, match="invalid argument"):
+                run()
+            continue
+        run()
+        torch.cuda.synchronize()
+        ref = out if ref is None else ref
+        assert torch.equal(out, ref)
+    tol = TOL64 if prec == "fp64" else TOL32
+    f = (lambda a: a) if prec == "fp64" else (lambda a: a.astype(np.float32).astype(np.float64))
+    assert oracle.rel_maxdiff(host(ref), oracle.bk5(nq, E, dbasis, f(g6i), f(u))) < tol
