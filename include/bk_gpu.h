@@ -99,9 +99,9 @@ typedef struct bk_options {
                             (its default), that default, or those of about
                             128 columns, 32, 15, 8, 6, 4, 3, 2, 2 for p =
                             1..8 (FP64 storage 1 at p = 7, 8), which is its
-                            default but for FP32 storage with G in the
-                            column layout (32, 7, 4, 5, 3, 1, 1, 1); other
-                            values BK_ERR_ARG.  The sweep kernels use
+                            default but for FP32 storage with six factors
+                            in the column layout (32, 7, 4, 5, 3, 1, 1, 1);
+                            other values BK_ERR_ARG.  The sweep kernels use
                             per-order tables measured on GB300 and ignore
                             it */
     int kernel;    /* bk_kernel_shape (BK5); BK1/BK3 have the sweep kernel only */

@@ -139,8 +139,10 @@ struct GlobalCol {
 // optional mass at the batch's first element in global memory.  after_s2()
 // runs (by every thread) right after the second barrier, once the staged data
 // are no longer read.  VEC: vb and mb start on 16 bytes, whole columns move as
-// vector accesses and the mass is loaded with G, ahead of the derivatives
-// (GlobalCol; for the FP32-storage forms).
+// vector accesses where their bytes allow it (GlobalCol), and with GDIR the mass
+// is loaded with G, ahead of the derivatives.  For the FP32-storage forms with
+// six factors: with nine the registers are short (mixed p=6 6.1 -> 7.8 us at
+// 0.45 M points).
 template <class Eng, int Q, int F, int LAYOUT, bool GDIR, bool VEC = false, class AfterS2>
 __device__ __forceinline__ void bk5_col_batch(const typename Eng::C* __restrict__ Dp, const typename Eng::V* Ds,
                                               const typename Eng::S* ub, const typename Eng::S* gb,
@@ -287,7 +289,11 @@ __device__ __forceinline__ void bk5_col_batch(const typename Eng::C* __restrict_
 #pragma unroll
             for (int k = 0; k < Q; ++k) Eng::vmadd(ay[k], dy, row[k]);
         }
-        S vcol[Q];
+        // where G is staged, columns that do not move as vectors are stored value
+        // by value as they come (held back, odd Q lost up to 7 %: mixed p=4,
+        // interleaved 29.2 -> 31.4 us at 2.2 M points)
+        constexpr bool kHold = GlobalCol<S, Q, VEC>::kVec || (VEC && GDIR);
+        S vcol[kHold ? Q : 1];
         const S* mo = (mb != nullptr) ? mb + el * Q3 + c * Q : nullptr;
 #pragma unroll
         for (int k = 0; k < Q; ++k) {
@@ -313,9 +319,10 @@ __device__ __forceinline__ void bk5_col_batch(const typename Eng::C* __restrict_
                 Eng::vmadd(am, m, ucol[k]);
                 res = Eng::loose(am);
             }
-            vcol[k] = Eng::store(res);
+            if constexpr (kHold) vcol[k] = Eng::store(res);
+            else vb[el * Q3 + c * Q + k] = Eng::store(res);
         }
-        GlobalCol<S, Q, VEC>::store(vb + el * Q3 + c * Q, vcol);
+        if constexpr (kHold) GlobalCol<S, Q, VEC>::store(vb + el * Q3 + c * Q, vcol);
     }
 }
 
@@ -394,11 +401,12 @@ __global__ void __launch_bounds__(BK5ColCfg<Eng, Q, EB, F, NBUF, LAYOUT>::NT)
         const S* ub = (sb == 0) ? us_slot0 : us_slot1;
         const S* gb = (sb == 0) ? gs_slot0 : gs_slot1;
         if constexpr (Cfg::GDIR) gb = G + e0 * F * Q3;
-        bk5_col_batch<Eng, Q, F, LAYOUT, Cfg::GDIR, sizeof(S) == 4>(prm.D, Ds, ub, gb, UV, R0, R1, GT, ne, tid, nt, v + e0 * Q3,
-                                         (mass != nullptr) ? mass + e0 * Q3 : nullptr, lambda, [&]() {
-                                             const long long nb = bt + NBUF * stride;
-                                             if (nb < nbatch) issue(nb, sb);
-                                         });
+        bk5_col_batch<Eng, Q, F, LAYOUT, Cfg::GDIR, sizeof(S) == 4 && F == 6>(
+            prm.D, Ds, ub, gb, UV, R0, R1, GT, ne, tid, nt, v + e0 * Q3, (mass != nullptr) ? mass + e0 * Q3 : nullptr,
+            lambda, [&]() {
+                const long long nb = bt + NBUF * stride;
+                if (nb < nbatch) issue(nb, sb);
+            });
     }
 }
 

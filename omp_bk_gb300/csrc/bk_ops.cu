@@ -226,19 +226,21 @@ int bk5_sweep_q(int F, const double* D, long long E, const void* u, const void* 
 // Column kernel: stage buffers.  With G read straight from HBM (FP32 storage,
 // column layout) only u is staged, and one buffer leaves room for more blocks
 // (q = 6 with the mass term 230 -> 224 us, q = 4 180 -> 177); the FP32-storage
-// forms of the other layouts take two, the FP64 engines, ALU-bound, one.
+// forms of the other layouts, and of nine factors, take two, the FP64 engines,
+// ALU-bound, one.
 constexpr bool col_gdir() { return sizeof(typename Eng::S) == 4 && BK_LAYOUT_TU == 2; }
-constexpr int col_nbuf() { return (sizeof(typename Eng::S) == 4 && !col_gdir()) ? 2 : 1; }
+constexpr int col_nbuf(int f) { return sizeof(typename Eng::S) == 4 && !(col_gdir() && f == 6) ? 2 : 1; }
 // Elements per block: about 128 columns.
 constexpr int col_eb_128(int q) { return (q * q >= 64) ? ((sizeof(typename Eng::S) == 4) ? 2 : 1) : (128 + q * q - 1) / (q * q); }
-// The default: with G straight from HBM the fastest measured at about 2^25
-// points with the mass term (us, about 128 columns -> this): q = 3 265 -> 252,
-// q = 4 188 -> 177, q = 5 250 -> 241, q = 6 240 -> 224, q = 7 281 -> 265, q = 8
-// 234 -> 210, q = 9 362 -> 318.
-constexpr int col_eb(int q)
+// The default: with six factors straight from HBM the fastest measured at about
+// 2^25 points with the mass term (us, about 128 columns -> this): q = 3 265 ->
+// 252, q = 4 188 -> 177, q = 5 250 -> 241, q = 6 240 -> 224, q = 7 281 -> 265,
+// q = 8 234 -> 210, q = 9 362 -> 318.  Not with nine factors, whose loads bound
+// the blocks otherwise.
+constexpr int col_eb(int q, int f)
 {
     constexpr int t[8] = {32, 7, 4, 5, 3, 1, 1, 1};   // q = 2..9
-    return col_gdir() ? t[q - 2] : col_eb_128(q);
+    return col_gdir() && f == 6 ? t[q - 2] : col_eb_128(q);
 }
 
 template <int Q, int EB, int F, int LAYOUT, int NBUF>
@@ -264,20 +266,16 @@ int bk5col_f(int F, int eb, const double* D, long long E, const void* u, const v
              double lambda, void* v, cudaStream_t s)
 {
     // the option names the default or about 128 columns, and gets what it names
-    constexpr int NB = col_nbuf();
-    constexpr int EB0 = col_eb(Q);
+    constexpr int NB = col_nbuf(6);
+    constexpr int EB0 = col_eb(Q, 6);
     constexpr int EB1 = col_eb_128(Q);
-    if (eb == 0) eb = EB0;
-    if (eb != EB0 && eb != EB1) return BK_ERR_ARG;
-    if (F == 6) {
-        if (eb == EB0) return bk5col_q<Q, EB0, 6, BK_LAYOUT_TU, NB>(D, E, u, G, mass, lambda, v, s);
-        return bk5col_q<Q, EB1, 6, BK_LAYOUT_TU, NB>(D, E, u, G, mass, lambda, v, s);
-    }
-    if (F == 9) {
-        if (eb == EB0) return bk5col_q<Q, EB0, 9, BK_LAYOUT_TU, NB>(D, E, u, G, mass, lambda, v, s);
-        return bk5col_q<Q, EB1, 9, BK_LAYOUT_TU, NB>(D, E, u, G, mass, lambda, v, s);
-    }
-    return BK_ERR_PREC;
+    static_assert(col_eb(Q, 9) == EB1, "nine factors have one number");
+    if (F != 6 && F != 9) return BK_ERR_PREC;
+    if (eb == 0) eb = F == 6 ? EB0 : EB1;
+    if (eb != EB1 && (F == 9 || eb != EB0)) return BK_ERR_ARG;
+    if (F == 9) return bk5col_q<Q, EB1, 9, BK_LAYOUT_TU, col_nbuf(9)>(D, E, u, G, mass, lambda, v, s);
+    if (eb == EB0) return bk5col_q<Q, EB0, 6, BK_LAYOUT_TU, NB>(D, E, u, G, mass, lambda, v, s);
+    return bk5col_q<Q, EB1, 6, BK_LAYOUT_TU, NB>(D, E, u, G, mass, lambda, v, s);
 }
 #endif  // BK_OP_TU == 6
 
