@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(BK3AdjCfg<Eng, Q, EB, DPAR>::NT)
     const S* ks = nullptr;
     auto issue_ur = [&](long long bt, bool arrive) {
         const long long e0 = bt * EB;
-        const int ne = batch_elems<EB, S>(E, e0);
+        const int ne = batch_elems<Eng, EB, EO>(E, e0);
         uint32_t tx = 0;
         if (tid == 0) fence_proxy_async();
         us = stage_issue<S>(ustage, u + e0 * P3, ne * P3, u + E * P3, bar, tx, tid, nt);
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(BK3AdjCfg<Eng, Q, EB, DPAR>::NT)
     };
     auto issue_gk = [&](long long bt) {
         const long long e0 = bt * EB;
-        const int ne = batch_elems<EB, S>(E, e0);
+        const int ne = batch_elems<Eng, EB, EO>(E, e0);
         uint32_t tx = 0;
         if (tid == 0) fence_proxy_async();
         gs = stage_issue<GS>(gstage, G + e0 * 6 * Q3, ne * 6 * Q3, G + E * 6 * Q3, bar, tx, tid, nt);
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(BK3AdjCfg<Eng, Q, EB, DPAR>::NT)
     uint32_t phase = 0;
     for (long long bt = blockIdx.x < nbatch ? blockIdx.x : -1; bt >= 0; bt = walk.next, phase ^= 1u) {
         const long long e0 = bt * EB;
-        const int ne = batch_elems<EB, S>(E, e0);
+        const int ne = batch_elems<Eng, EB, EO>(E, e0);
         if (walk.start(phase, ctx, tid)) return;
         // g_u -> (W1, W2, W3) with W0 as scratch; g_res -> (W4, W5, W6), W6 = W0
         // (its last use) unless DPAR

@@ -779,13 +779,17 @@ __device__ __forceinline__ bool batch_wait_failed(uint64_t* bar, uint32_t phase,
 // (the loops over elements vanish).  For FP32 storage (S) the compiler is told
 // the range, so that a loop over lines that the block's threads cover in one
 // step is none (BK1 p=1 176 -> 158 us, BK3 p=4 228 -> 220); the float-float
-// kernels were slower with it (adjoint p=4 729 -> 754, BK5 p=8 890 -> 950).
-template <int EB, class S>
+// kernels were slower with it (adjoint p=4 729 -> 754, BK5 p=8 890 -> 950), and
+// so are BK1's general contractions (RANGE false; FP32 p=3 at 6 M points 29.1 ->
+// 35.5 us).  Float-float with the general contractions is not told of EB = 1
+// (ONE false; adjoint p=5 50 -> 58 us at 0.45 M points) but where that costs the
+// registers of a second block (BK3 p=7 803 -> 1114 at 6 M, BK5 p=8 448 -> 624).
+template <class Eng, int EB, bool ONE, bool RANGE = true>
 __device__ __forceinline__ int batch_elems(long long E, long long e0)
 {
-    if (EB == 1) return 1;
+    if (EB == 1 && (ONE || Eng::kId != BK_ENGINE_FF)) return 1;
     const int ne = int((E - e0) < EB ? (E - e0) : EB);
-    if constexpr (sizeof(S) == 4) __builtin_assume(ne >= 1 && ne <= EB);
+    if constexpr (sizeof(typename Eng::S) == 4 && RANGE) __builtin_assume(ne >= 1 && ne <= EB);
     return ne;
 }
 
@@ -1290,7 +1294,7 @@ __global__ void __launch_bounds__(BK5Cfg<Eng, Q, EB, F, LAYOUT, DPAR>::NT, BK5Cf
     //    batch bt's phase completes when both have landed
     auto issue_g = [&](long long bt) {
         const long long e0 = bt * EB;
-        const int ne = batch_elems<EB, S>(E, e0);
+        const int ne = batch_elems<Eng, EB, EO || Q == 9>(E, e0);
         uint32_t tx = 0;
         if (tid == 0) fence_proxy_async();
         gs = stage_issue<GS>(smem + Cfg::U_BYTES, G + e0 * F * Q3, ne * F * Q3, G + E * F * Q3, bar, tx, tid, nt);
@@ -1298,7 +1302,7 @@ __global__ void __launch_bounds__(BK5Cfg<Eng, Q, EB, F, LAYOUT, DPAR>::NT, BK5Cf
     };
     auto issue_u = [&](long long bt) {
         const long long e0 = bt * EB;
-        const int ne = batch_elems<EB, S>(E, e0);
+        const int ne = batch_elems<Eng, EB, EO || Q == 9>(E, e0);
         uint32_t tx = 0;
         if (tid == 0) fence_proxy_async();
         us = stage_issue<S>(smem, u + e0 * Q3, ne * Q3, u + E * Q3, bar, tx, tid, nt);
@@ -1312,7 +1316,7 @@ __global__ void __launch_bounds__(BK5Cfg<Eng, Q, EB, F, LAYOUT, DPAR>::NT, BK5Cf
     for (long long bt = blockIdx.x < nbatch ? blockIdx.x : -1; bt >= 0; bt = walk.next, phase ^= 1u) {
         if (walk.start(phase, ctx, tid)) return;
         const long long e0 = bt * EB;
-        const int ne = batch_elems<EB, S>(E, e0);
+        const int ne = batch_elems<Eng, EB, EO || Q == 9>(E, e0);
         const S* mb = (mass != nullptr) ? mass + e0 * Q3 : nullptr;
         const S* ub = us;
         const GS* gb = gs;
@@ -1392,7 +1396,7 @@ __global__ void __launch_bounds__(BK1Cfg<Eng, Q, EB>::NT)
     const S* js = nullptr;
     auto issue = [&](long long bt) {
         const long long e0 = bt * EB;
-        const int ne = batch_elems<EB, S>(E, e0);
+        const int ne = batch_elems<Eng, EB, EO, EO>(E, e0);
         uint32_t tx = 0;
         if (tid == 0) fence_proxy_async();
         us = stage_issue<S>(ustage, u + e0 * P3, ne * P3, u + E * P3, bar, tx, tid, nt);
@@ -1403,7 +1407,7 @@ __global__ void __launch_bounds__(BK1Cfg<Eng, Q, EB>::NT)
     uint32_t phase = 0;
     for (long long bt = blockIdx.x < nbatch ? blockIdx.x : -1; bt >= 0; bt = walk.next, phase ^= 1u) {
         const long long e0 = bt * EB;
-        const int ne = batch_elems<EB, S>(E, e0);
+        const int ne = batch_elems<Eng, EB, EO, EO>(E, e0);
         if (walk.start(phase, ctx, tid)) return;
         if constexpr (EO) {   // B centro-symmetric (GLL nodes, Gauss points)
             if constexpr (kDirectIO) {
@@ -1548,7 +1552,7 @@ __global__ void __launch_bounds__(BK3Cfg<Eng, Q, EB, DPAR>::NT)
     const S* ks = nullptr;
     auto issue = [&](long long bt) {
         const long long e0 = bt * EB;
-        const int ne = batch_elems<EB, S>(E, e0);
+        const int ne = batch_elems<Eng, EB, EO || Q == 9>(E, e0);
         uint32_t tx = 0;
         if (tid == 0) fence_proxy_async();
         us = stage_issue<S>(ustage, u + e0 * P3, ne * P3, u + E * P3, bar, tx, tid, nt);
@@ -1560,7 +1564,7 @@ __global__ void __launch_bounds__(BK3Cfg<Eng, Q, EB, DPAR>::NT)
     uint32_t phase = 0;
     for (long long bt = blockIdx.x < nbatch ? blockIdx.x : -1; bt >= 0; bt = walk.next, phase ^= 1u) {
         const long long e0 = bt * EB;
-        const int ne = batch_elems<EB, S>(E, e0);
+        const int ne = batch_elems<Eng, EB, EO || Q == 9>(E, e0);
         if (walk.start(phase, ctx, tid)) return;
         // fluxes (k G grad u with the coefficient); written twice, with and
         // without k, so that no point carries predicated-off products

@@ -104,6 +104,18 @@ constexpr int adj_eb(int q)
     return q == 3 ? 14 : q == 4 ? 8 : q == 5 ? 5 : q == 6 ? 3 : 1;
 }
 
+// The general contractions (matrices without the symmetry): elements per block
+// of their own where the tables above, measured with the even-odd ones, lose (us
+// at 25 M points with them -> with these: float-float BK3 q = 7 1962 -> 1581,
+// FP32 BK1 q = 6 156 -> 147, q = 7 173 -> 151; float-float BK1 q = 9 at 0.06 M
+// points 11.6 -> 10.4).
+constexpr int gen_eb1(int q)
+{
+    if (eng_is_ff()) return default_eb(q);
+    return q == 6 || q == 7 ? default_eb(q) : sweep_eb1(q);
+}
+constexpr int gen_eb3(int q) { return eng_is_ff() && q == 7 ? 3 : sweep_eb3(q); }
+
 // Sets the dynamic shared-memory size of a kernel on the current device once
 // and returns its resident blocks per SM (0 if it cannot run).  Tag makes the
 // cache one per kernel instantiation (kernels of one signature share K).
@@ -280,12 +292,10 @@ int bk5col_f(int F, int eb, const double* D, long long E, const void* u, const v
 #endif  // BK_OP_TU == 6
 
 #if BK_OP_TU == 1
-template <int Q, int EB>
+template <int Q>
 int bk1_q(const double* B, long long E, const void* jxw, const void* u, void* v, int jxw_t, cudaStream_t s)
 {
-    using Cfg = BK1Cfg<Eng, Q, EB>;
     using S = typename Eng::S;
-    static_assert(Cfg::SMEM <= 232448, "BK1 block exceeds the shared memory of an SM");
     P13<typename Eng::C, Q> prm;
     for (int i = 0; i < (Q - 1) * Q; ++i) prm.B[i] = Eng::coef(B[i]);
     for (int i = 0; i < Q * Q; ++i) prm.D[i] = Eng::coef(0.0);
@@ -295,6 +305,9 @@ int bk1_q(const double* B, long long E, const void* jxw, const void* u, void* v,
                     make_eor<typename Eng::C, Q - 1, Q>(B, Q, false, +1, prm.bb, &Eng::coef);
     auto go = [&](auto e) {
         constexpr bool EO = decltype(e)::value;
+        constexpr int EB = EO ? sweep_eb1(Q) : gen_eb1(Q);
+        using Cfg = BK1Cfg<Eng, Q, EB>;
+        static_assert(Cfg::SMEM <= 232448, "BK1 block exceeds the shared memory of an SM");
         return launch_walk<Cfg, EO, EB>(&bk1_kernel<Eng, Q, EB, EO, false>, &bk1_kernel<Eng, Q, EB, EO, EO>, E, s, prm, E,
                                         static_cast<const S*>(u), static_cast<const S*>(jxw), jxw_t,
                                         static_cast<S*>(v));
@@ -349,7 +362,7 @@ int bk3_q(const double* B, const double* D, long long E, const void* G, const vo
         return bk3_launch<Q, DP ? sweep_eb3_dpar(Q) : EB, true, DP>(prm, E, G, k, u, v, s);
     }
     if (gform != BK_G_STORAGE) return BK_ERR_PREC;   // split G: even-odd B and D (GLL nodes, Gauss points)
-    return bk3_launch<Q, EB, false, 0>(prm, E, G, k, u, v, s);
+    return bk3_launch<Q, gen_eb3(Q), false, 0>(prm, E, G, k, u, v, s);
 }
 
 #endif  // BK_OP_TU == 3
@@ -445,14 +458,14 @@ int BK_CAT(launch_bk1, BK_SFX)(int p, long long E, const double* B, const void* 
 {
     (void)eb;
     switch (p + 2) {
-        case 3: return bk1_q<3, sweep_eb1(3)>(B, E, jxw, u, v, jxw_t, s);
-        case 4: return bk1_q<4, sweep_eb1(4)>(B, E, jxw, u, v, jxw_t, s);
-        case 5: return bk1_q<5, sweep_eb1(5)>(B, E, jxw, u, v, jxw_t, s);
-        case 6: return bk1_q<6, sweep_eb1(6)>(B, E, jxw, u, v, jxw_t, s);
-        case 7: return bk1_q<7, sweep_eb1(7)>(B, E, jxw, u, v, jxw_t, s);
-        case 8: return bk1_q<8, sweep_eb1(8)>(B, E, jxw, u, v, jxw_t, s);
-        case 9: return bk1_q<9, sweep_eb1(9)>(B, E, jxw, u, v, jxw_t, s);
-        case 10: return bk1_q<10, sweep_eb1(10)>(B, E, jxw, u, v, jxw_t, s);
+        case 3: return bk1_q<3>(B, E, jxw, u, v, jxw_t, s);
+        case 4: return bk1_q<4>(B, E, jxw, u, v, jxw_t, s);
+        case 5: return bk1_q<5>(B, E, jxw, u, v, jxw_t, s);
+        case 6: return bk1_q<6>(B, E, jxw, u, v, jxw_t, s);
+        case 7: return bk1_q<7>(B, E, jxw, u, v, jxw_t, s);
+        case 8: return bk1_q<8>(B, E, jxw, u, v, jxw_t, s);
+        case 9: return bk1_q<9>(B, E, jxw, u, v, jxw_t, s);
+        case 10: return bk1_q<10>(B, E, jxw, u, v, jxw_t, s);
         default: return BK_ERR_ORDER;
     }
 }
