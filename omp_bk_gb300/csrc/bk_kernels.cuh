@@ -450,7 +450,7 @@ __device__ __forceinline__ void sweep_eo(const typename Eng::V* in, typename Eng
 // strides are computed, not constants, so that one code body serves all
 // three directions.  LOOSE: the outputs as unevaluated pairs (sum_diff_loose),
 // for sweeps whose outputs are only summed next (the transposed derivatives).
-template <class Eng, class WB, int Q, bool LOOSE = false, class EM>
+template <class Eng, class WB, int Q, bool LOOSE = false, bool MID = false, class EM>
 __device__ __forceinline__ void sweep_eo_dyn(const typename Eng::V* in, typename Eng::V* out, int ne, const EM& m,
                                              int tid, int nt, int dir)
 {
@@ -492,7 +492,7 @@ __device__ __forceinline__ void sweep_eo_dyn(const typename Eng::V* in, typename
             A t = Eng::first(m.r[0], Eng::odd(lw[0]));
 #pragma unroll
             for (int n = 1; n < H; ++n) Eng::madd(t, m.r[n], Eng::odd(lw[n]));
-            po[H * SD] = Eng::result(t);
+            po[H * SD] = LOOSE && MID ? Eng::loose(t) : Eng::result(t);
         }
     }
 }
@@ -972,7 +972,8 @@ struct BK5Cfg {
 // latency-bound float-float arithmetic gets more warps per SM.  DPAR = 1:
 // one code body per direction (strides known at compile time); DPAR = 2: one
 // body for all three, the direction's strides in registers (a third of the
-// instruction footprint of the stage).
+// instruction footprint of the stage); DPAR = 3: that body with the middle point
+// of an odd line loose too, as one thread per line leaves it (the same bits).
 struct SyncOnly {
     __device__ __forceinline__ bool operator()() const
     {
@@ -1044,7 +1045,7 @@ __device__ __forceinline__ bool bk5_sweep_batch(const typename Eng::C* __restric
     __syncthreads();
     // 3. gradient: qr -> W0 (along i), qs -> W1 (along j), qt (along k) ->
     //    QT (in place into W2 after the other two have read it unless DPAR)
-    if constexpr (DPAR == 2) {
+    if constexpr (DPAR >= 2) {
         if (grp < 3) sweep_eo_dyn<Eng, WB, Q>(W2, grp == 0 ? W0 : (grp == 1 ? W1 : W3), ne, eo, tg, ntd, grp);
     } else if constexpr (DPAR == 1) {
         if (grp == 0) sweep_eo<Eng, WB, 0, Q>(W2, W0, ne, eo, tg, ntd);
@@ -1118,11 +1119,11 @@ __device__ __forceinline__ bool bk5_sweep_batch(const typename Eng::C* __restric
     if (after_pw()) return true;   // the G stage (and u, without a mass term) is free from here
     // 5. transposed derivatives, in place: along i on W0, along j on W1 and
     //    (even-odd) along k on QT
-    if constexpr (DPAR == 2) {
+    if constexpr (DPAR >= 2) {
         if (grp < 3) {
             // summed in the last pass, never multiplied: loose pairs
             V* Wg = grp == 0 ? W0 : (grp == 1 ? W1 : W3);
-            sweep_eo_dyn<Eng, WB, Q, true>(Wg, Wg, ne, eot, tg, ntd, grp);
+            sweep_eo_dyn<Eng, WB, Q, true, DPAR == 3>(Wg, Wg, ne, eot, tg, ntd, grp);
         }
     } else if constexpr (DPAR == 1) {
         if (grp == 0) sweep_eo<Eng, WB, 0, Q, true>(W0, W0, ne, eot, tg, ntd);

@@ -169,6 +169,56 @@ int launch_walk(K sk, K dk, long long E, cudaStream_t s, const Args&... args)
     return cudaGetLastError() == cudaSuccess ? BK_OK : BK_ERR_CUDA;
 }
 
+// The shapes above were measured on launches of many waves.  One of a few waves
+// ends with its fullest SM, so a second shape of fewer elements, or of the
+// direction groups (which share an element's lines among three times the threads
+// and so are done sooner where an SM has little to do), is kept beside a large
+// one, and taken for up to `few` batches of the large shape per SM, and from
+// there to kFewPerSm where the elements that the fullest SM has room for times
+// the cost of an element are fewer.  cost: of an element in the second shape
+// where both fill the chip, in per cent of one in the large shape; 0: no second
+// shape.  Both give the same bits.  Measured at 26 sizes of each shape (5e3 to
+// 4e6 points) against the large shape alone: float-float BK5 q = 6 0.73 to 0.82
+// of its time below 1.3 batches per SM, q = 7 0.57 to 0.9 up to three, BK3 q = 6
+// 0.81 below one and 0.82 at 3.7, q = 5 0.94, BK1 q = 9 0.80 to 0.95, adjoint q =
+// 5 0.87 to 0.95; FP32 adjoint q = 5 and 6 0.91, BK1 q = 6 and 7 0.91 to 0.99.
+struct Few {
+    int eb, dpar, few, cost;
+};
+constexpr int kFewPerSm = 24;
+constexpr Few kNoFew{1, 0, 0, 0};
+constexpr Few few5(int q)
+{
+    return !eng_is_ff() ? kNoFew : q == 6 ? Few{4, 2, 1, 102} : q == 7 ? Few{2, 3, 3, 103} : kNoFew;
+}
+constexpr Few few3(int q)
+{
+    return !eng_is_ff() ? kNoFew : q == 5 ? Few{8, 0, 0, 110} : q == 6 ? Few{3, 2, 4, 104} : kNoFew;
+}
+constexpr Few few1(int q)
+{
+    if (eng_is_dfma()) return kNoFew;
+    if (eng_is_ff()) return q == 9 ? Few{2, 0, 0, 110} : kNoFew;
+    return q == 6 ? Few{4, 0, 0, 105} : q == 7 ? Few{3, 0, 0, 103} : kNoFew;
+}
+constexpr Few few_adj(int q)
+{
+    if (eng_is_dfma()) return kNoFew;
+    if (eng_is_ff()) return q == 5 ? Few{3, 0, 0, 102} : kNoFew;
+    return q == 5 ? Few{3, 0, 0, 107} : q == 6 ? Few{2, 0, 0, 103} : kNoFew;
+}
+
+// Whether the second shape f is taken instead of the large one (eb elements per
+// block).
+inline bool take_few(long long E, int eb, const Few& f)
+{
+    const long long sms = sm_count();
+    auto batches = [&](int n) { return (E + n - 1) / n; };
+    auto room = [&](int n) { return (batches(n) + sms - 1) / sms * n; };   // of the fullest SM
+    if (batches(eb) > kFewPerSm * sms) return false;
+    return batches(eb) <= f.few * sms || room(f.eb) * f.cost <= room(eb) * 100;
+}
+
 #if BK_OP_TU == 5
 // One launch of bk5_kernel with the given shape.
 // GS: the type G is stored in (the storage type, or ff2 pairs split ahead of
@@ -220,12 +270,20 @@ int bk5_sweep_q(int F, const double* D, long long E, const void* u, const void* 
     if (eo) {
         constexpr int DP = sweep_dpar5(Q);
         constexpr int EB = fit_eb5<Q, 6, DP ? sweep_eb5_dpar(Q) : sweep_eb5(Q), DP>();
+        // gs: G as stored, or split ahead of time (the float-float engine)
+        auto go = [&](auto gs) {
+            using GS = decltype(gs);
+            if constexpr (few5(Q).cost > 0) {
+                if (take_few(E, EB, few5(Q)))
+                    return bk5_launch<Q, few5(Q).eb, 6, L, true, few5(Q).dpar, GS>(prm, E, u, G, mass, lambda, v, s);
+            }
+            return bk5_launch<Q, EB, 6, L, true, DP, GS>(prm, E, u, G, mass, lambda, v, s);
+        };
         if (gform == BK_G_FF) {
-            // G split ahead of time: the float-float engine's even-odd path
-            if constexpr (eng_is_ff()) return bk5_launch<Q, EB, 6, L, true, DP, ff2>(prm, E, u, G, mass, lambda, v, s);
+            if constexpr (eng_is_ff()) return go(ff2{});
             return BK_ERR_PREC;
         }
-        return bk5_launch<Q, EB, 6, L, true, DP>(prm, E, u, G, mass, lambda, v, s);
+        return go(typename Eng::S{});
     }
     if (gform != BK_G_STORAGE) return BK_ERR_PREC;   // split G: even-odd D (GLL points), 6 factors
     if (F == 6) return bk5_launch<Q, fit_eb5<Q, 6, sweep_eb5(Q)>(), 6, L, false, 0>(prm, E, u, G, mass, lambda, v, s);
@@ -303,16 +361,22 @@ int bk1_q(const double* B, long long E, const void* jxw, const void* u, void* v,
     // Gauss points)
     const bool eo = make_eor<typename Eng::C, Q, Q - 1>(B, Q, true, +1, prm.bi, &Eng::coef) &&
                     make_eor<typename Eng::C, Q - 1, Q>(B, Q, false, +1, prm.bb, &Eng::coef);
-    auto go = [&](auto e) {
+    auto go = [&](auto e, auto n) {
         constexpr bool EO = decltype(e)::value;
-        constexpr int EB = EO ? sweep_eb1(Q) : gen_eb1(Q);
+        constexpr int EB = decltype(n)::value;
         using Cfg = BK1Cfg<Eng, Q, EB>;
         static_assert(Cfg::SMEM <= 232448, "BK1 block exceeds the shared memory of an SM");
         return launch_walk<Cfg, EO, EB>(&bk1_kernel<Eng, Q, EB, EO, false>, &bk1_kernel<Eng, Q, EB, EO, EO>, E, s, prm, E,
                                         static_cast<const S*>(u), static_cast<const S*>(jxw), jxw_t,
                                         static_cast<S*>(v));
     };
-    return eo ? go(std::true_type{}) : go(std::false_type{});
+    using Large = std::integral_constant<int, sweep_eb1(Q)>;
+    if (!eo) return go(std::false_type{}, std::integral_constant<int, gen_eb1(Q)>{});
+    if constexpr (few1(Q).cost > 0) {
+        if (take_few(E, Large::value, few1(Q)))
+            return go(std::true_type{}, std::integral_constant<int, few1(Q).eb>{});
+    }
+    return go(std::true_type{}, Large{});
 }
 
 #endif  // BK_OP_TU == 1
@@ -353,13 +417,21 @@ int bk3_q(const double* B, const double* D, long long E, const void* G, const vo
     const bool eo = make_p13_eo<typename Eng::C, Q>(prm, B, D, &Eng::coef);
     if (eo) {
         constexpr int DP = sweep_dpar3(Q) ? 2 : 0;
+        constexpr int EBL = DP ? sweep_eb3_dpar(Q) : EB;
+        // gs: G as stored, or split ahead of time (the float-float engine)
+        auto go = [&](auto gs) {
+            using GS = decltype(gs);
+            if constexpr (few3(Q).cost > 0) {
+                if (take_few(E, EBL, few3(Q)))
+                    return bk3_launch<Q, few3(Q).eb, true, few3(Q).dpar, GS>(prm, E, G, k, u, v, s);
+            }
+            return bk3_launch<Q, EBL, true, DP, GS>(prm, E, G, k, u, v, s);
+        };
         if (gform == BK_G_FF) {
-            // G split ahead of time: the float-float engine's even-odd path
-            if constexpr (eng_is_ff())
-                return bk3_launch<Q, DP ? sweep_eb3_dpar(Q) : EB, true, DP, ff2>(prm, E, G, k, u, v, s);
+            if constexpr (eng_is_ff()) return go(ff2{});
             return BK_ERR_PREC;
         }
-        return bk3_launch<Q, DP ? sweep_eb3_dpar(Q) : EB, true, DP>(prm, E, G, k, u, v, s);
+        return go(typename Eng::S{});
     }
     if (gform != BK_G_STORAGE) return BK_ERR_PREC;   // split G: even-odd B and D (GLL nodes, Gauss points)
     return bk3_launch<Q, gen_eb3(Q), false, 0>(prm, E, G, k, u, v, s);
@@ -395,13 +467,20 @@ int bk3adj_q(const double* B, const double* D, long long E, const void* G, const
     for (int i = 0; i < Q * Q; ++i) prm.D[i] = Eng::coef(D[i]);
     if (make_p13_eo<typename Eng::C, Q>(prm, B, D, &Eng::coef)) {
         constexpr int DP = adj_dpar(Q) ? 2 : 0;
+        // gs: G as stored, or split ahead of time (the float-float engine)
+        auto go = [&](auto gs) {
+            using GS = decltype(gs);
+            if constexpr (few_adj(Q).cost > 0) {
+                if (take_few(E, EB, few_adj(Q)))
+                    return bk3adj_launch<Q, few_adj(Q).eb, true, few_adj(Q).dpar, GS>(prm, E, G, k, u, res, dk, dG, s);
+            }
+            return bk3adj_launch<Q, EB, true, DP, GS>(prm, E, G, k, u, res, dk, dG, s);
+        };
         if (gform == BK_G_FF) {
-            // G split ahead of time: the float-float engine's even-odd path
-            if constexpr (eng_is_ff())
-                return bk3adj_launch<Q, EB, true, DP, ff2>(prm, E, G, k, u, res, dk, dG, s);
+            if constexpr (eng_is_ff()) return go(ff2{});
             return BK_ERR_PREC;
         }
-        return bk3adj_launch<Q, EB, true, DP>(prm, E, G, k, u, res, dk, dG, s);
+        return go(typename Eng::S{});
     }
     if (gform != BK_G_STORAGE) return BK_ERR_PREC;
     return bk3adj_launch<Q, EB, false, 0>(prm, E, G, k, u, res, dk, dG, s);

@@ -684,3 +684,65 @@ def test_bk5_column_elements_per_block(bklib, prec, layout, p):
     tol = TOL64 if prec == "fp64" else TOL32
     f = (lambda a: a) if prec == "fp64" else (lambda a: a.astype(np.float32).astype(np.float64))
     assert oracle.rel_maxdiff(host(ref), oracle.bk5(nq, E, dbasis, f(g6i), f(u))) < tol
+
+
+WALKS = [("bk1", "fp64", "pqr"), ("bk1", "fp64", "rqp"), ("bk1", "mixed", "pqr"), ("bk1", "fp32", "rqp"),
+         ("bk3", "fp64", ""), ("bk3", "fp64", "k"), ("bk3", "fp64", "split"), ("bk3", "fp64", "split k"),
+         ("bk3", "mixed", "k"), ("bk3", "fp32", ""), ("bk5", "fp64", "column"), ("bk5", "fp64", "factor mass"),
+         ("bk5", "fp64", "column mass"), ("bk5", "fp64", "column split mass"), ("bk5", "mixed", "column mass"),
+         ("bk5", "mixed", "factor"), ("adjoint", "fp64", ""), ("adjoint", "fp64", "split"), ("adjoint", "mixed", "")]
+
+
+@pytest.mark.parametrize("p", P_ALL)
+@pytest.mark.parametrize("op,prec,form", WALKS)
+def test_launch_sizes_agree(bklib, op, prec, form, p):
+    """The same 840 elements over and over (840 is a multiple of every number of
+    elements a block takes), in launches of all kinds: 840 elements, at most 840
+    batches, fewer than eight per SM, are dealt to the blocks; a few thousand take
+    the shapes for launches of a few waves and those of many; and with 40000
+    batches and more (no SM holds more than 32 blocks) the blocks take over one
+    another's.  Every repetition to the bit, the last one partial."""
+    q = p + 1 if op == "bk5" else p + 2
+    nb, nu, nq = 840, (p + 1) ** 3, q ** 3
+    dt = torch.float64 if prec == "fp64" else torch.float32
+    pr = {"fp64": bklib.PREC_FP64, "fp32": bklib.PREC_FP32, "mixed": bklib.PREC_MIXED}[prec]
+    gen = torch.Generator(device="cuda").manual_seed(7 * p + WALKS.index((op, prec, form)))
+    rnd = lambda n, lo: (torch.rand(nb, n, generator=gen, device="cuda", dtype=torch.float64) + lo).to(dt)
+    u, res, w, G = rnd(nu, -0.5), rnd(nu, -0.5), rnd(nq, 0.5), rnd(6 * nq, 0.1)
+    B, D = bklib.bk1_bk3_matrices(p)[:2]
+    D5 = bklib.bk5_matrices(p)[0]
+    split = bklib.G_FF if "split" in form else bklib.G_STORAGE
+    lay = bklib.LAYOUT_FACTOR if "factor" in form else bklib.LAYOUT_COLUMN
+
+    def run(E):
+        many = lambda x: x.expand(-(-E // nb), *x.shape).reshape(-1, x.shape[1])[:E].contiguous()
+        eu = many(u)
+        v = torch.full_like(eu, float("nan"))
+        if op == "bk1":
+            bklib.bk1_apply(p, E, B, many(w), eu, v, prec=pr,
+                            jxw_layout=bklib.JXW_RQP if form == "rqp" else bklib.JXW_PQR)
+            return [v]
+        g = many(G)
+        if "split" in form:
+            g = bklib.g_to_ff(g.reshape(-1))
+        if op == "bk3":
+            bklib.bk3_apply(p, E, B, D, g, eu, v, k=many(w) if "k" in form else None, prec=pr, gform=split)
+            return [v]
+        if op == "bk5":
+            bklib.bk5_apply(p, E, D5, g, eu, v, prec=pr, layout=lay, kernel=bklib.KERNEL_SWEEP,
+                            mass=many(w) if "mass" in form else None, lam=0.75, gform=split)
+            return [v]
+        dk, dG = (torch.full((E, n), float("nan"), dtype=dt, device="cuda") for n in (nq, 6 * nq))
+        bklib.bk3_adjoint(p, E, B, D, g, many(w), eu, many(res), dk, dG, prec=pr, gform=split)
+        return [dk, dG]
+
+    base = run(nb)
+    torch.cuda.synchronize()
+    assert not any(torch.isnan(b).any() for b in base)
+    eb = min(16, max(1, 256 // q ** 2))   # at least a block's elements
+    for E in (nb + 1, 2 * nb + 17, 5 * nb + 3, 12 * nb + 1, 40000 * eb + 11):
+        for out, b in zip(run(E), base):
+            n = E // nb
+            assert torch.equal(out[:n * nb].reshape(n, nb, -1), b.expand(n, *b.shape))
+            assert torch.equal(out[n * nb:], b[:E - n * nb])
+            del out
