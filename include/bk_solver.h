@@ -25,7 +25,10 @@ typedef struct bk_order_range {
     int elems_per_tile;  /* elements per tile of the persistent launch, with
                             elems_per_tile * q^2 <= 1024 (the column body:
                             <= 256, one thread per column); 0: the library's
-                            own (28, 16, 5, 3, 2, 2, 1 for p = 2..8) */
+                            own for p = 2..8: 28, 16, 5, 3, 2, 2, 1 (the
+                            column body with FP32 storage 28, 16, 6, 4, 3, 2,
+                            2), and 14, 8, 5, 3, 2, 2, 1 in a plan that would
+                            have fewer tiles than the device has SMs */
 } bk_order_range;
 
 typedef struct bk_hplan* bk_hplan_t;
@@ -42,7 +45,9 @@ int bk_hplan_destroy(bk_hplan_t plan);
  * 4, 5: shared memory per block of the sweep body's launch for FP64 / FP32
  * storage (a launch needs at most 232448 bytes); 6, 7: the threads and G
  * staging set by bk_hplan_set_shape; 8, 9: the tiles and threads of the
- * FP64-storage launches (bk_hplan_set_fp64_shape). */
+ * FP64-storage launches (bk_hplan_set_fp64_shape); 10: the tiles of the column
+ * body with FP32 storage; 11, 12: the threads (of a direction group, FP64) that
+ * the sweep body's FP32 and FP64 launches have. */
 long long bk_hplan_size(bk_hplan_t plan, int what);
 
 /* The body of the persistent launch: BK_KERNEL_SWEEP (line sweeps in the
@@ -54,8 +59,8 @@ int bk_hplan_set_kernel(bk_hplan_t plan, int kernel);
 
 /* The shape of the even-odd sweep body's persistent launch.  threads: per
  * block, a multiple of 32 in 64..256, or 0 (the default) for the largest
- * tile's lines (elements x q^2, at most 128); tiles with more lines than
- * threads loop over their lines, so tile sizes per order and the block are
+ * tile's lines (elements x q^2), at most 256, or at most 128 where every range
+ * has the library's own tiles; tiles with more lines than threads loop over their lines, so tile sizes per order and the block are
  * chosen apart.  The FP64 launch runs three thread groups of that size (one
  * per direction).  gstage (FP32 storage): 1 stages each tile's G into shared
  * memory by TMA, 0 (the default) reads it in the pointwise stage straight

@@ -143,7 +143,7 @@ struct GlobalCol {
 // is loaded with G, ahead of the derivatives.  For the FP32-storage forms with
 // six factors: with nine the registers are short (mixed p=6 6.1 -> 7.8 us at
 // 0.45 M points).
-template <class Eng, int Q, int F, int LAYOUT, bool GDIR, bool VEC = false, class AfterS2>
+template <class Eng, int Q, int F, int LAYOUT, bool GDIR, bool VEC = false, bool HOLD = true, class AfterS2>
 __device__ __forceinline__ void bk5_col_batch(const typename Eng::C* __restrict__ Dp, const typename Eng::V* Ds,
                                               const typename Eng::S* ub, const typename Eng::S* gb,
                                               typename Eng::V* UV, typename Eng::V* R0, typename Eng::V* R1,
@@ -289,10 +289,11 @@ __device__ __forceinline__ void bk5_col_batch(const typename Eng::C* __restrict_
 #pragma unroll
             for (int k = 0; k < Q; ++k) Eng::vmadd(ay[k], dy, row[k]);
         }
-        // where G is staged, columns that do not move as vectors are stored value
-        // by value as they come (held back, odd Q lost up to 7 %: mixed p=4,
-        // interleaved 29.2 -> 31.4 us at 2.2 M points)
-        constexpr bool kHold = GlobalCol<S, Q, VEC>::kVec || (VEC && GDIR);
+        // columns that do not move as vectors may be stored value by value as they
+        // come (!HOLD): faster in the single-order kernel where G is staged (mixed
+        // p=4, interleaved, 2.2 M points 31.4 -> 29.2 us), slower in the mixed-order
+        // one (mixed p=8, 1.5 M points 27.3 -> 30.0)
+        constexpr bool kHold = HOLD || GlobalCol<S, Q, VEC>::kVec || (VEC && GDIR);
         S vcol[kHold ? Q : 1];
         const S* mo = (mb != nullptr) ? mb + el * Q3 + c * Q : nullptr;
 #pragma unroll
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(BK5ColCfg<Eng, Q, EB, F, NBUF, LAYOUT>::NT)
         const S* ub = (sb == 0) ? us_slot0 : us_slot1;
         const S* gb = (sb == 0) ? gs_slot0 : gs_slot1;
         if constexpr (Cfg::GDIR) gb = G + e0 * F * Q3;
-        bk5_col_batch<Eng, Q, F, LAYOUT, Cfg::GDIR, sizeof(S) == 4 && F == 6>(
+        bk5_col_batch<Eng, Q, F, LAYOUT, Cfg::GDIR, sizeof(S) == 4 && F == 6, false>(
             prm.D, Ds, ub, gb, UV, R0, R1, GT, ne, tid, nt, v + e0 * Q3, (mass != nullptr) ? mass + e0 * Q3 : nullptr,
             lambda, [&]() {
                 const long long nb = bt + NBUF * stride;

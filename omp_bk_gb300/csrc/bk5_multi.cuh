@@ -210,6 +210,7 @@ struct PMultiEO {
     MultiSeg seg[kMultiNQ];
     int nseg;
     int block;      // threads per block (0: the largest tile's lines)
+    int named;      // the caller named elements per tile
     int gstage;     // FP32 storage: G staged by TMA (1) or read from global memory (0)
     long long n;    // values of u, v and mass over all segments
     long long ng;   // values of G over all segments

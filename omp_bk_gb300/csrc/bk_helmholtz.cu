@@ -35,7 +35,7 @@ namespace {
 
 constexpr int kDynWaves = 8;   // tiles per resident block from which a launch shares them dynamically
 constexpr int kNT = 256;   // threads per block of the persistent kernel (per thread group), at most
-constexpr int kDefThreads = 128;  // threads of the sweep launch (per group) unless the plan sets them
+constexpr int kDefThreads = 128;  // threads of the sweep launch (per group) with the default tiles
 constexpr int kMaxTileLines = 1024;   // lines (elements x q^2) of a tile, at most
 // Elements per tile of the orders p = 2..8 unless the plan sets them: the
 // autotuner's picks at 5 M to 43 M points, mixed and float-float, but 28
@@ -44,6 +44,16 @@ constexpr int kMaxTileLines = 1024;   // lines (elements x q^2) of a tile, at mo
 // largest tile's lines, p = 2..8, 43.5 M points: mixed 414 -> 340 us,
 // float-float 2494 -> 1550.
 constexpr int kDefTile[7] = {28, 16, 5, 3, 2, 2, 1};
+// Those of a plan with fewer tiles than SMs, which the larger tiles of p = 2 and
+// 3 would only make longer: what fits kDefThreads lines (p = 2, 3, 6.6e3 points:
+// mixed 4.0 -> 3.2 us, float-float 7.1 -> 5.1, 1.1e5 points: mixed 4.1 -> 3.5).
+constexpr int kDefTileFew[7] = {14, 8, 5, 3, 2, 2, 1};
+// Those of the column body with FP32 storage, whose blocks have kNT threads
+// whatever the tile: at p = 4..8 as many columns as that body was measured with
+// (us with kDefTile -> this, mixed: p = 4..8, 20 M points 343 -> 316, p = 8, 6 M
+// points 114 -> 88).  FP64 storage keeps kDefTile (float-float, p = 4..8, 20 M
+// points 1408 against 1907).
+constexpr int kDefTileCol[7] = {28, 16, 6, 4, 3, 2, 2};
 constexpr int kRedBlocks = 1216;   // 8 blocks of 256 threads per SM
 constexpr int kMaxDotParts = 4864;  // blocks of the persistent launch at most (32 per SM)
 constexpr int kRedThreads = 256;
@@ -121,8 +131,8 @@ struct MultiLaunch {
 };
 
 // The even-odd sweep launch: blockDim = the largest tile's lines (eb q^2),
-// rounded up to whole warps, or the plan's block size (kDefThreads by default)
-// when that is smaller
+// rounded up to whole warps, or the plan's block size when that is smaller
+// (kDefThreads with the default tiles, kNT with tiles that the caller named)
 // (the sweeps of a tile with more lines than threads loop over them); three
 // times that with direction-parallel groups (DPAR); MAXT threads at most,
 // MINB blocks per SM asked of the register allocator.  GST: FP32 G staged.
@@ -132,14 +142,14 @@ struct MultiEOLaunch {
     // dot product (its partials are summed in a fixed order), nor in the forms
     // that only a tuned plan or the DFMA engine takes
     static constexpr bool kDyn = !DOT && !GST && Eng::kId != BK_ENGINE_DFMA;
-    static int threads(const MultiSeg* seg, int nseg, int block)
+    static int threads(const PMultiEO<typename Eng::C>& prm)
     {
         int nt = 64;
-        for (int s = 0; s < nseg; ++s) {
-            const int l = (seg[s].eb * seg[s].q * seg[s].q + 31) / 32 * 32;
+        for (int s = 0; s < prm.nseg; ++s) {
+            const int l = (prm.seg[s].eb * prm.seg[s].q * prm.seg[s].q + 31) / 32 * 32;
             nt = l > nt ? l : nt;
         }
-        const int most = block > 0 ? block : kDefThreads;
+        const int most = prm.block > 0 ? prm.block : prm.named ? kNT : kDefThreads;
         if (nt > most) nt = most;
         if (DPAR) nt *= 3;
         return nt > MAXT ? MAXT : nt;
@@ -181,7 +191,7 @@ struct MultiEOLaunch {
         int ub = 0, gb = 0, wb = 0;
         const int total = smem(prm, ub, gb, wb);
         if (total > 232448) return 0;
-        return prepare(total, threads(prm.seg, prm.nseg, prm.block));
+        return prepare(total, threads(prm));
     }
     // dot_part (optional): one partial sum of u . v per block, their count in
     // *nparts; skip (with it, optional): the launch does nothing if *skip is not 0
@@ -192,7 +202,7 @@ struct MultiEOLaunch {
         using S = typename Eng::S;
         int ub = 0, gb = 0, wb = 0;
         const int total = smem(prm, ub, gb, wb);
-        const int nt = threads(prm.seg, prm.nseg, prm.block);
+        const int nt = threads(prm);
         if (total > 232448) return BK_ERR_ARG;
         if (DOT != (dot_part != nullptr)) return BK_ERR_ARG;
         auto kern = bk5_multi_eo_kernel<Eng, MAXT, MINB, DOT, DPAR, GST>;
@@ -634,6 +644,9 @@ struct bk_hplan {
     // NULL: the plan's tiles)
     MultiTile* tiles64;
     int ntiles64;
+    // the column body's tiles with FP32 storage (NULL: the plan's)
+    MultiTile* tilesc;
+    int ntilesc;
     bool shaped;        // the caller named elements per tile
     long long n;        // values of a vector
     long long ng;       // values of G
@@ -772,9 +785,12 @@ int apply_plan(bk_hplan* h, int eng, const void* G, const void* mass, double lam
     switch (eng) {
         case 0: return MultiLaunch<EngDfma, 1>::run(h->p_dfma, h->tiles, h->ntiles, u, G, mass, lambda, v, s);
         case 1: return MultiLaunch<EngFF, 1>::run(h->p_ff, h->tiles, h->ntiles, u, G, mass, lambda, v, s);
-        case 2: return MultiLaunch<EngF32, 2>::run(h->p_f32, h->tiles, h->ntiles, u, G, mass, lambda, v, s);
-        default: return MultiLaunch<EngMixed, 2>::run(h->p_f32, h->tiles, h->ntiles, u, G, mass, lambda, v, s);
+        default: break;
     }
+    const MultiTile* tc = h->tilesc ? h->tilesc : h->tiles;
+    const int nc = h->tilesc ? h->ntilesc : h->ntiles;
+    if (eng == 2) return MultiLaunch<EngF32, 2>::run(h->p_f32, tc, nc, u, G, mass, lambda, v, s);
+    return MultiLaunch<EngMixed, 2>::run(h->p_f32, tc, nc, u, G, mass, lambda, v, s);
 }
 
 int ck(cudaError_t e) { return e == cudaSuccess ? BK_OK : BK_ERR_CUDA; }
@@ -783,8 +799,10 @@ int ck(cudaError_t e) { return e == cudaSuccess ? BK_OK : BK_ERR_CUDA; }
 // columns (elements x q^2) must fit one block.
 bool column_fits(const bk_hplan& h)
 {
-    for (int s = 0; s < h.nseg; ++s)
-        if (h.seg[s].eb * h.seg[s].q * h.seg[s].q > kNT) return false;
+    for (int s = 0; s < h.nseg; ++s) {
+        const int q = h.seg[s].q;
+        if (h.seg[s].eb * q * q > kNT || h.p_f32.seg[s].eb * q * q > kNT) return false;
+    }
     return true;
 }
 
@@ -940,6 +958,18 @@ int bk_hplan_create(bk_hplan_t* out, int norders, const bk_order_range* orders, 
     std::memset(h->seg, 0, sizeof(h->seg));
     h->device = current_device();
     h->nseg = norders;
+    // the default tiles
+    long long ndef = 0;
+    for (int s = 0; s < norders; ++s) {
+        const int p = orders[s].p, eb = orders[s].elems_per_tile;
+        if (p < kMultiQmin - 1 || p > kMultiQmax - 1 || orders[s].E <= 0) continue;   // (refused below, or empty)
+        const int n = eb > 0 ? eb : kDefTile[p - 2];
+        ndef += (orders[s].E + n - 1) / n;
+    }
+    const int* def = ndef < sm_count() ? kDefTileFew : kDefTile;
+    const int* defc = def == kDefTile ? kDefTileCol : def;
+    int ebc[kMultiNQ];
+    bool own = false;   // the column body has tiles of its own
     long long uo = 0, go = 0;
     for (int s = 0; s < norders; ++s) {
         const int p = orders[s].p;
@@ -950,7 +980,9 @@ int bk_hplan_create(bk_hplan_t* out, int norders, const bk_order_range* orders, 
         const int q = p + 1;
         int eb = orders[s].elems_per_tile;
         if (eb > 0) h->shaped = true;
-        if (eb <= 0) eb = kDefTile[p - 2];
+        ebc[s] = eb > 0 ? eb : defc[p - 2];
+        if (eb <= 0) eb = def[p - 2];
+        own = own || ebc[s] != eb;
         if (eb * q * q > kMaxTileLines || orders[s].E < 0 || !D[s]) {
             delete h;
             return orders[s].E < 0 ? BK_ERR_SIZE : BK_ERR_ARG;
@@ -972,6 +1004,10 @@ int bk_hplan_create(bk_hplan_t* out, int norders, const bk_order_range* orders, 
     fill_params(h->p_f32, *h, D, conv_f);
     h->eo_ok = fill_eo_params(h->e_dfma, *h, D, conv_d) && fill_eo_params(h->e_ff, *h, D, conv_ff) &&
                fill_eo_params(h->e_f32, *h, D, conv_f);
+    h->e_dfma.named = h->e_ff.named = h->e_f32.named = h->shaped;
+    for (int s = 0; s < norders; ++s) h->p_f32.seg[s].eb = ebc[s];
+    const std::vector<MultiTile> col = own ? make_tiles(h->p_f32.seg, norders) : std::vector<MultiTile>();
+    h->ntilesc = int(col.size());
     h->kernel = h->eo_ok ? BK_KERNEL_SWEEP : BK_KERNEL_COLUMN;
     if (!h->eo_ok && !column_fits(*h)) {
         delete h;
@@ -990,8 +1026,11 @@ int bk_hplan_create(bk_hplan_t* out, int norders, const bk_order_range* orders, 
     rc |= ck(cudaMalloc(&h->part, 8 * (kRedBlocks > kMaxDotParts ? kRedBlocks : kMaxDotParts)));
     rc |= ck(cudaMalloc(&h->sc, 8 * S_NSCAL));
     rc |= ck(cudaMalloc(&h->rpart, 8 * kCgBlocks));
+    if (own) rc |= ck(cudaMalloc(&h->tilesc, sizeof(MultiTile) * (col.size() + 1)));
     if (rc == BK_OK && h->ntiles > 0)
         rc = ck(cudaMemcpyAsync(h->tiles, h->htiles.data(), sizeof(MultiTile) * h->ntiles, cudaMemcpyHostToDevice, s));
+    if (rc == BK_OK && h->ntilesc > 0)
+        rc = ck(cudaMemcpyAsync(h->tilesc, col.data(), sizeof(MultiTile) * col.size(), cudaMemcpyHostToDevice, s));
     if (rc == BK_OK) rc = ck(cudaStreamSynchronize(s));
     if (rc != BK_OK) {
         bk_hplan_destroy(h);
@@ -1007,6 +1046,7 @@ int bk_hplan_destroy(bk_hplan_t h)
     free_graph(h);
     cudaFree(h->tiles);
     cudaFree(h->tiles64);
+    cudaFree(h->tilesc);
     cudaFree(h->r64);
     cudaFree(h->r32);
     cudaFree(h->p32);
@@ -1036,6 +1076,9 @@ long long bk_hplan_size(bk_hplan_t h, int what)
     if (what == 7) return h->e_f32.gstage;
     if (what == 8) return h->tiles64 ? h->ntiles64 : h->ntiles;
     if (what == 9) return h->e_ff.block;
+    if (what == 10) return h->tilesc ? h->ntilesc : h->ntiles;
+    if (what == 11) return MultiEOLaunch<EngMixed, 256, 4>::threads(h->e_f32);
+    if (what == 12) return MultiFF::threads(h->e_ff) / 3;
     return -1;
 }
 
@@ -1080,6 +1123,7 @@ int bk_hplan_set_fp64_shape(bk_hplan_t h, const int* elems_per_tile, int threads
     h->ntiles64 = ntiles;
     for (int s = 0; s < h->nseg; ++s) h->e_dfma.seg[s].eb = h->e_ff.seg[s].eb = seg[s].eb;
     h->e_dfma.block = h->e_ff.block = elems_per_tile ? threads : h->e_f32.block;
+    h->e_dfma.named = h->e_ff.named = h->shaped || elems_per_tile != nullptr;
     return BK_OK;
 }
 

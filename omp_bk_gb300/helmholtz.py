@@ -4,7 +4,8 @@ include/bk_solver.h.
 
 Elements of each order p are stored one order after another (u, v, mass:
 E_p (p+1)^3 values; G: E_p 6 (p+1)^3 values in the column layout).  One
-persistent launch applies the operator to all orders; the solver's inner
+persistent launch applies the operator to all orders (a large float-float
+apply of a plan at default shapes: a launch per order); the solver's inner
 FP32 CG runs as one CUDA graph (conditional WHILE node) per refinement step.
 """
 from __future__ import annotations
@@ -62,9 +63,13 @@ def _declare():
 
 
 def default_tiles(p: int) -> int:
-    """Elements per tile when no tuning is given (the library's own default),
-    p = 2..8."""
-    return (28, 16, 5, 3, 2, 2, 1)[p - 2]
+    """Elements per tile when no tuning is given: the library's own default for
+    a plan with a tile per SM and more, p = 2..8 (other orders, which no plan
+    has: about 128 lines of (p+1) points, at least one element)."""
+    q2 = (p + 1) ** 2
+    if 2 <= p <= 8:
+        return (28, 16, 5, 3, 2, 2, 1)[p - 2]
+    return 1 if q2 >= 100 else (128 + q2 - 1) // q2
 
 
 class HelmholtzPlan:
@@ -103,8 +108,9 @@ class HelmholtzPlan:
 
     def set_shape(self, block: int = 0, gstage: int = 0):
         """Threads per block of the sweep body's launch (0: the largest
-        tile's lines, at most 128; tiles with more lines loop over them) and, for FP32
-        storage, whether G is staged in shared memory (bk_hplan_set_shape)."""
+        tile's lines, at most 256, or 128 with the library's own tiles; tiles
+        with more lines loop over them) and, for FP32 storage, whether G is
+        staged in shared memory (bk_hplan_set_shape)."""
         check(_declare().bk_hplan_set_shape(self.h, int(block), int(gstage)), "bk_hplan_set_shape")
 
     def set_fp64_shape(self, tiles=None, block: int = 0, stream=None):

@@ -520,3 +520,51 @@ def test_cg_scaled_operator(bklib, small_plan):
     (n1, x1), (n2, x2) = res.values()
     assert n1 == n2 and 10 < n1 < 2000
     assert float(torch.linalg.norm(x1 - x2) / torch.linalg.norm(x1)) < 1e-9
+
+
+@pytest.mark.parametrize("form", ["many", "few", "named", "fp64 named"])
+def test_default_tiles_and_threads(bklib, form):
+    """The library's own tiles, of the sweep body and of the column body with
+    FP32 storage, for plans of many and of few tiles, and the threads of launches
+    without a block: at most 128 with them, the largest tile's lines up to 256
+    with tiles that the caller named.  Every body's apply against the orders'."""
+    from omp_bk_gb300 import helmholtz
+    bk = bklib
+    E = [(p, 61 if form == "few" else 1501) for p in range(2, 9)]
+    own = {2: 28, 3: 16, 4: 5, 5: 3, 6: 2, 7: 2, 8: 1}
+    col = {2: 28, 3: 16, 4: 6, 5: 4, 6: 3, 7: 2, 8: 2}
+    if form == "few":
+        own = col = {2: 14, 3: 8, 4: 5, 5: 3, 6: 2, 7: 2, 8: 1}
+        E = E[:3]
+    else:
+        assert [helmholtz.default_tiles(p) for p in own] == list(own.values())
+    if form == "named":
+        own = col = {p: max(1, 200 // (p + 1) ** 2) for p in own}
+        E = [(p, n, own[p]) for p, n in E]
+    plan = helmholtz.HelmholtzPlan(E)
+    size = lambda what: bk.lib().bk_hplan_size(plan.h, what)
+    count = lambda t: sum(-(-o[1] // t[o[0]]) for o in E)
+    lines = lambda t: max(-(-t[o[0]] * (o[0] + 1) ** 2 // 32) * 32 for o in E)
+    try:
+        if form == "fp64 named":
+            t64 = {p: max(1, 200 // (p + 1) ** 2) for p in own}
+            plan.set_fp64_shape(t64)
+            assert plan.fp64_ntiles == count(t64) and size(12) == lines(t64) > 128
+            plan.set_fp64_shape(None)
+        assert plan.ntiles == plan.fp64_ntiles == count(own) and size(10) == count(col)
+        most = 256 if form == "named" else 128
+        assert size(11) == size(12) == min(most, lines(own))
+        G, M = plan.geometry(seed=5)
+        u = bk.fill_uniform(torch.empty(plan.n, dtype=torch.float64, device="cuda"), 6)
+        for kern in (bk.KERNEL_SWEEP, bk.KERNEL_COLUMN):
+            plan.set_kernel(kern)
+            for prec in ("ff", "mixed", "fp32"):
+                _check_per_order(bk, plan, G, M, u, prec)
+    finally:
+        plan.close()
+
+
+@pytest.mark.parametrize("p,n", [(0, 128), (1, 32), (9, 1), (12, 1)])
+def test_default_tiles_of_other_orders(p, n):
+    from omp_bk_gb300.helmholtz import default_tiles
+    assert default_tiles(p) == n
