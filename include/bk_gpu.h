@@ -143,7 +143,9 @@ enum bk_kernel_shape {
                              all intermediates in shared memory */
     BK_KERNEL_COLUMN = 2  /* one thread per k-column of an element, the
                              k-direction and the pointwise products in
-                             registers, TMA double buffering */
+                             registers; u and G double-buffered by TMA, or u
+                             alone in one buffer and G from HBM to registers
+                             (FP32 storage, six factors, column layout) */
 };
 
 /* bk_options with the defaults: prec FP64, engine AUTO, BK5 layout

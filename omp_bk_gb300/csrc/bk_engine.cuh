@@ -73,8 +73,6 @@ struct EngDfma {
     __device__ static __forceinline__ V result(A acc) { return acc; }
     __device__ static __forceinline__ V loose(A acc) { return acc; }
     __device__ static __forceinline__ V mul(V a, V b) { return a * b; }
-    __device__ static __forceinline__ V vadd(V a, V b) { return a + b; }
-    __device__ static __forceinline__ V vsub(V a, V b) { return a - b; }
     struct V2 {
         V x, y;
     };
@@ -136,8 +134,6 @@ struct EngFF {
     // for values that are only summed or stored next: not renormalised
     __device__ static __forceinline__ V loose(A acc) { return acc_loose(acc); }
     __device__ static __forceinline__ V mul(V a, V b) { return ff_mul(a, b); }
-    __device__ static __forceinline__ V vadd(V a, V b) { return ff_add(a, b); }
-    __device__ static __forceinline__ V vsub(V a, V b) { return ff_add(a, ff{-b.hi, -b.lo}); }
     using V2 = ffp;
     using A2 = ffaccp;
     // operands of multiply-adds only: not renormalised
@@ -202,8 +198,6 @@ struct EngF32 {
     __device__ static __forceinline__ V result(A acc) { return acc; }
     __device__ static __forceinline__ V loose(A acc) { return acc; }
     __device__ static __forceinline__ V mul(V a, V b) { return a * b; }
-    __device__ static __forceinline__ V vadd(V a, V b) { return a + b; }
-    __device__ static __forceinline__ V vsub(V a, V b) { return a - b; }
     using V2 = f2;
     using A2 = f2;
     __device__ static __forceinline__ V2 even_odd(V a, V b) { return f2_make(a + b, a - b); }

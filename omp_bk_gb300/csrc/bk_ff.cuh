@@ -21,7 +21,8 @@
 // into a truncated 24-bit hi and the remaining 29 mantissa bits (rounded to a
 // float) with integer operations and one I2F; join() adds the lo part to the
 // bit pattern of hi as a count of double ulps.  Kernels send every other value
-// through join_fp64() instead, on the otherwise idle pipe.  Values outside [2^-74, 2^128) (split) or [2^-74, 2^127) (join) take a slow
+// through join_fp64() instead, on the otherwise idle pipe: the same bits.
+// Values outside [2^-74, 2^128) (split) or [2^-74, 2^127) (join) take a slow
 // path through the FP64 pipe.
 //
 // Every operation uses the __f*_rn intrinsics, which the compiler never
@@ -190,17 +191,6 @@ __device__ __forceinline__ void acc_sum_diff_loose(const ffacc& a, const ffacc& 
     two_sum(b.s, -a.s, diff.hi, f);
     sum.lo = __fadd_rn(e, __fadd_rn(a.c, b.c));
     diff.lo = __fadd_rn(f, __fsub_rn(b.c, a.c));
-}
-
-// a + b, both float-float, normalised (TwoSum of the hi parts, lo parts added).
-__device__ __forceinline__ ff ff_add(const ff a, const ff b)
-{
-    float s, e;
-    two_sum(a.hi, b.hi, s, e);
-    e = __fadd_rn(e, __fadd_rn(a.lo, b.lo));
-    ff r;
-    fast_two_sum(s, e, r.hi, r.lo);
-    return r;
 }
 
 // ---- packed FP32: two lanes per instruction -----------------------------------

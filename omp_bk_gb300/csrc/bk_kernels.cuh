@@ -115,8 +115,8 @@ constexpr int bk3_box(int q, int vbytes, int what)   // what: 0 ZP, 1 PS, 2 elem
 // (j = 0..7 at each of 4 i) otherwise meets rows j and j + 4 in the same
 // banks; swapping the two halves of every row whose j has bit 2 set makes
 // the 128-bit k-line accesses (VEC) and, with PS = 8 mod 32, the j-direction
-// sweeps conflict-free.  Only BK3's FP32-storage forms at Q = 8 use it
-// (box_model.py --op 32): the model's wavefronts per element fall from 612
+// sweeps conflict-free.  BK3's and BK1's FP32-storage forms at Q = 8 use it
+// (BK3: box_model.py --op 32): the model's wavefronts per element fall from 612
 // to 474, its shared-memory instructions from 424 to 344, and BK3 p=6 mixed
 // went from 110.2 to 120.1 GDoF/s (same results).
 constexpr int bk3_swz(int q, int vbytes) { return (q == 8 && vbytes == 4) ? 4 : 0; }
@@ -1259,8 +1259,8 @@ __device__ __forceinline__ bool bk5_sweep_batch(const typename Eng::C* __restric
     return false;
 }
 
-// The block goes from batch to batch (Walk).  One stage buffer: the next batch's u and G are copied into it as soon as the current batch
-// stops reading them (after the pointwise stage; u after the last pass when a
+// The block goes from batch to batch (Walk).  One stage buffer: the next batch's
+// u and G are copied into it as soon as the current batch stops reading them (after the pointwise stage; u after the last pass when a
 // mass term reads it there), so the copies overlap the transposed sweeps and
 // the last pass instead of stalling the block at the start of each batch.
 template <class Eng, int Q, int EB, int F, int LAYOUT, bool EO = false, int DPAR = 0, class GS = typename Eng::S,
@@ -1354,7 +1354,7 @@ struct BK1Cfg {
     static constexpr int Q3 = Q * Q * Q;
     static constexpr int P3 = P * P * P;
     static constexpr int NT = ((EB * Q * Q + 31) / 32) * 32 < 64 ? 64 : ((EB * Q * Q + 31) / 32) * 32;
-    static constexpr int U_BYTES = stage_bytes<S>(EB * Q3);   // also holds the P^3 output
+    static constexpr int U_BYTES = stage_bytes<S>(EB * Q3);   // (u's P^3 values an element need less)
     static constexpr int J_BYTES = stage_bytes<S>(EB * Q3);
     static constexpr int W_BYTES = ((2 * EB * WB::size * int(sizeof(V)) + 15) / 16) * 16;
     static constexpr int SMEM = U_BYTES + J_BYTES + W_BYTES + kTailBytes;

@@ -59,7 +59,8 @@ namespace BK_TU_NS {
 constexpr int default_eb(int q) { return (q * q >= 100) ? 1 : ((q * q >= 64) ? 2 : (128 + q * q - 1) / (q * q)); }
 
 // Elements per block of the even-odd kernels, the fastest measured per engine
-// and q on GB300 at 2^23..2^26 points per apply.  A sweep gives each thread a
+// and q on GB300 at 2^23..2^26 points per apply, with the batches dealt (Walk;
+// shared dynamically, BK3's q = 8 was measured again and moved).  A sweep gives each thread a
 // line, so an EB whose EB q^2 lines just fill whole warps leaves no thread
 // idle: q = 3: 7 or 14 (63, 126 lines), q = 5: 5 (125), q = 6: 7 (252),
 // q = 7: 5 (245).  Where fewer elements per block let more blocks share an
@@ -148,6 +149,8 @@ int grid_for(long long nbatch, int occ)
 // dealt / dynamic: BK5 p=4 float-float at 2, 4, 8, 16 waves 18.7 / 20.5, 35.1 /
 // 37.0, 64.8 / 64.3, 125 / 120 us; BK3 p=5 FP32 at 4, 8, 15 waves 24.8 / 23.2,
 // 45.4 / 45.2, 85.7 / 82.1.
+// One line for all: float-float loses below it, and FP32 storage, which these
+// figures would let share from 4 on, gives up at most a tenth there.
 constexpr int kDynWaves = 8;
 
 // One launch of a batch kernel: dealt (sk) or dynamic (dk) by the batches per
